@@ -1619,6 +1619,8 @@ struct Batched {
 	cudaEvent_t ev = nullptr;
 	Tuning tuned;
 	EstState est;
+	Resident *res = nullptr;       // grids that fit on chip: whole solves in one launch, dense vectors
+	const double *rhs = nullptr;   // right-hand sides of the running batch (resident: b or the caller's)
 	std::vector<int> lane_res;  // result codes of the batch being processed
 	double *t_acc = nullptr, *q_acc = nullptr;
 	int period = 32;
@@ -1975,6 +1977,8 @@ int batched_alloc(Ctx *c) {
 	}
 	B->g0_host = B->gl_host + 1;
 	B->lane_res.assign(B->R, 0);
+	const int rrc = resident_alloc(c, B->ks, B->mixed, B->R, &B->res);
+	if (rrc) return rrc;
 	bind_impl(B);
 	// The zero-fills must be complete before a caller stream (sedi_set_stream) uses the buffers.
 	if (cudaStreamSynchronize(c->stream) != cudaSuccess) return set_cuda_error(c, cudaGetLastError(), "batched_alloc");
@@ -2013,6 +2017,7 @@ size_t batched_bytes(int solver, int precision, int batch, long long n1, long lo
 	size_t total = nT * up(elems * ts) + up(elems * xs) + up(elems * 8) * (mixed ? 2 : 1);
 	total += up(sizeof(double) * nblk * kMaxDots * R) + 3 * up(1) + up(sizeof(double) * kLaneDoubles * R) +
 	         up(sizeof(int) * 5 * R) + 2 * up(sizeof(double) * g.n);
+	if (g.n1 <= 512 && g.n <= (1 << 22)) total += 12 * up(1);  // the resident solver's face rows and reduction words
 	return total;
 }
 
@@ -2037,6 +2042,7 @@ static void free_batched(Batched *B) {
 void batched_free(Ctx *c) {
 	Batched *B = (Batched *)c->batched;
 	if (!B) return;
+	resident_free(B->res);
 	void *ptrs[] = {B->x, B->xh, B->b, B->r, B->p0, B->p1, B->partials, B->ticket, B->gl, B->lane_mem, B->lane_int,
 	                B->t_acc, B->q_acc, B->w[0], B->w[1], B->u, B->q, B->sv, B->z, B->r1, B->v[0], B->v[1],
 	                B->rhat};
@@ -2356,7 +2362,47 @@ struct Impl {
 	}
 };
 
+// The resident solver's setup and chunk: the launch solves the whole batch,
+// so no lane is active after it.
+static int resident_setup(Ctx *c, Batched *B, int nrhs, int maxiter, double tol) {
+	Global g0 = {};
+	g0.maxiter = maxiter;
+	g0.tol = tol;
+	g0.tol_in = B->mixed ? B->theta * tol : tol;
+	g0.period = B->period;
+	g0.nrhs = nrhs;
+	*B->g0_host = g0;
+	BTRY(cudaMemcpyAsync(B->gl, B->g0_host, sizeof(Global), cudaMemcpyHostToDevice, c->stream));
+	return 0;
+}
+
+static int resident_chunk(Ctx *c, Batched *B) {
+	const Global &g0 = *B->g0_host;
+	ResIO io = {};
+	io.lanes = g0.nrhs;
+	io.rhs = B->rhs;
+	io.x = B->mixed ? B->xh : (double *)B->x;
+	io.xlo = B->mixed ? B->x : nullptr;
+	io.tol = g0.tol;
+	io.tol_in = g0.tol_in;
+	io.maxiter = g0.maxiter;
+	io.period = g0.period;
+	io.o_err = B->ls.err;
+	io.o_bb = B->ls.bb;
+	io.o_rr = B->ls.rr;
+	io.o_exit = B->ls.exit_iter;
+	io.o_reason = B->ls.reason;
+	io.o_done = B->ls.done;
+	io.err = &B->gl->err;
+	return resident_launch(c, B->res, io);
+}
+
 static void bind_impl(Batched *B) {
+	if (B->res) {
+		B->setup_fn = resident_setup;
+		B->chunk_fn = resident_chunk;
+		return;
+	}
 	if (B->mixed) {  // FP64 fields in slices of mixed_slice_fp64 lanes
 		if (B->rbT == 4 && B->rbD == 4) {
 			B->setup_fn = Impl<float, 4, 4>::setup;
@@ -2668,6 +2714,17 @@ int batched_solve_dev(Ctx *c, int nrhs, const double *b, double *x, int maxiter,
 	}
 	cudaStream_t s = c->stream;
 	const long long n = c->g.n;
+	if (B->res) {  // dense vectors: b is read in place, x by way of the context's own (b and x may overlap)
+		double *const xd = B->mixed ? B->xh : (double *)B->x;
+		const size_t bytes = sizeof(double) * (size_t)n * nrhs;
+		B->rhs = b;
+		BTRY(cudaMemcpyAsync(xd, x, bytes, cudaMemcpyDeviceToDevice, s));
+		const int rc = batched_run_resident(c, nrhs, maxiter, tol, final_err, final_iter, results);
+		if (rc < 0) return rc;
+		BTRY(cudaMemcpyAsync(x, xd, bytes, cudaMemcpyDeviceToDevice, s));
+		BTRY(cudaStreamSynchronize(s));
+		return rc;
+	}
 	kb_interleave<<<blocks1d(n * B->R), 256, 0, s>>>(n, B->R, B->rbD, nrhs, b, B->b);
 	kb_interleave<<<blocks1d(n * B->R), 256, 0, s>>>(n, B->R, B->rbD, nrhs, x, B->mixed ? B->xh : (double *)B->x);
 	c->launches += 2;
@@ -2874,15 +2931,27 @@ static int est_start_batch(Ctx *c, Batched *B) {
 	cudaStream_t s = c->stream;
 	const long long n = c->g.n;
 	E.nb = E.samples - E.k0 < c->batch ? E.samples - E.k0 : c->batch;
-	if (E.probes_dev) {
-		kb_interleave<<<blocks1d(n * B->R), 256, 0, s>>>(n, B->R, B->rbD, E.nb, E.probes_dev + (size_t)E.k0 * n, B->b);
+	size_t x_elems = B->elems;
+	if (B->res) {  // dense vectors, no padding lanes; the caller's probes are read in place
+		x_elems = (size_t)n * E.nb;
+		B->rhs = E.probes_dev ? E.probes_dev + (size_t)E.k0 * n : B->b;
+		if (!E.probes_dev) {
+			if (device_fill_probes(E.seed + (uint32_t)E.k0, E.nb, n, 0, B->b, s))
+				return set_cuda_error(c, cudaGetLastError(), "device probes");
+			c->launches++;
+		}
 	} else {
-		if (E.nb < B->R) BTRY(cudaMemsetAsync(B->b, 0, B->elems * sizeof(double), s));  // padding lanes
-		if (device_fill_probes(E.seed + (uint32_t)E.k0, E.nb, n, B->rbD, B->b, s))
-			return set_cuda_error(c, cudaGetLastError(), "device probes");
+		B->rhs = B->b;
+		if (E.probes_dev) {
+			kb_interleave<<<blocks1d(n * B->R), 256, 0, s>>>(n, B->R, B->rbD, E.nb, E.probes_dev + (size_t)E.k0 * n, B->b);
+		} else {
+			if (E.nb < B->R) BTRY(cudaMemsetAsync(B->b, 0, B->elems * sizeof(double), s));  // padding lanes
+			if (device_fill_probes(E.seed + (uint32_t)E.k0, E.nb, n, B->rbD, B->b, s))
+				return set_cuda_error(c, cudaGetLastError(), "device probes");
+		}
+		c->launches++;
 	}
-	c->launches++;
-	BTRY(cudaMemsetAsync(B->mixed ? (void *)B->xh : B->x, 0, B->elems * sizeof(double), s));  // x = 0 (:175)
+	BTRY(cudaMemsetAsync(B->mixed ? (void *)B->xh : B->x, 0, x_elems * sizeof(double), s));  // x = 0 (:175)
 	int rc = B->setup_fn(c, B, E.nb, E.maxiter, E.tol);
 	if (!rc) rc = B->chunk_fn(c, B);
 	if (rc) return rc;
@@ -2974,7 +3043,7 @@ int batched_est_advance(Ctx *c, int *done) {
 		}
 		// Batch solved: lane results and t += x.*v, q += v.*v (:195, :198).
 		if ((rc = enqueue_lane_copy(c, B))) break;
-		kb_accumulate<<<blocks1d(n), 256, 0, s>>>(n, B->rbD, E.nb, B->mixed ? B->xh : (const double *)B->x, B->b,
+		kb_accumulate<<<blocks1d(n), 256, 0, s>>>(n, B->res ? 1 : B->rbD, E.nb, B->mixed ? B->xh : (const double *)B->x, B->rhs,
 		                                          B->t_acc, B->q_acc, E.first);
 		c->launches++;
 		E.first = false;

@@ -509,15 +509,19 @@ int plain_alloc(Ctx *c) {
 	SEDI_TRY(cudaMemsetAsync(c->ticket, 0, sizeof(unsigned), c->stream));  // ordered before the context's kernels
 	SEDI_TRY(cudaStreamSynchronize(c->stream));
 	SEDI_TRY(cudaMalloc(&c->st, sizeof(SolveState)));
+	SEDI_TRY(cudaMemsetAsync(c->st, 0, sizeof(SolveState), c->stream));
 	SEDI_TRY(cudaMallocHost(&c->st_host, sizeof(SolveState)));
 	c->hist_cap = 0;
 	c->hist = nullptr;
 	c->chunk_iters = 16;
-	return pairs_alloc(c);
+	const int rc = resident_alloc(c, c->solver, false, 1, &c->res);
+	return rc ? rc : pairs_alloc(c);
 }
 
 void plain_free(Ctx *c) {
 	pairs_free(c);
+	resident_free(c->res);
+	c->res = nullptr;
 	double *vecs[] = {c->x, c->b, c->iM, c->r, c->rhat, c->p[0], c->p[1], c->v[0], c->v[1],
 	                  c->w[0], c->w[1], c->u, c->q, c->s, c->z, c->t_acc, c->q_acc, c->partials, c->hist};
 	for (double *p : vecs)
@@ -633,6 +637,50 @@ static int finish_result(const Ctx *c, const SolveState &s, double *final_err, i
 	return 1;
 }
 
+// Result of the solve in c->st_host, and the length of its history.
+static int finish_solve(Ctx *c, int maxiter, double *final_err, int *final_iter) {
+	const SolveState st = *c->st_host;
+	// Entries written: hist[0] plus one per iteration that printed its err
+	// (the s-norm exit and the rho breakdown leave before printing).
+	if (st.reason == STOP_EARLY) c->hist_len = 1;
+	else if (st.reason == STOP_SNORM || st.reason == STOP_RHO) c->hist_len = st.exit_iter;
+	else c->hist_len = (st.exit_iter > maxiter ? maxiter : st.exit_iter) + 1;
+	return finish_result(c, st, final_err, final_iter);
+}
+
+// The whole solve in one launch (grids whose vectors fit on chip).
+static int resident_solve(Ctx *c, const double *b, double *x, int maxiter, double tol, double *final_err,
+                          int *final_iter) {
+	const int rc = ensure_hist(c, maxiter);
+	if (rc) return rc;
+	ResIO io = {};
+	io.lanes = 1;
+	io.rhs = b;
+	io.x = x;
+	io.tol = io.tol_in = tol;
+	io.maxiter = maxiter;
+	io.o_err = &c->st->err;
+	io.o_bb = &c->st->bb;
+	io.o_rr = &c->st->rr;
+	io.o_exit = &c->st->exit_iter;
+	io.o_reason = &c->st->reason;
+	io.o_done = &c->st->done;
+	io.hist = c->hist;
+	io.err = &c->st->wait_err;
+	const int e = resident_launch(c, c->res, io);
+	if (e) return e;
+	SEDI_TRY(cudaMemcpyAsync(c->st_host, c->st, sizeof(SolveState), cudaMemcpyDeviceToHost, c->stream));
+	SEDI_TRY(cudaStreamSynchronize(c->stream));
+	if (c->st_host->wait_err) {
+		SEDI_TRY(cudaMemsetAsync(c->st, 0, sizeof(SolveState), c->stream));
+		c->error = "resident solver timed out waiting for its blocks";
+		return SEDI_ERR_CUDA;
+	}
+	c->st_host->tol = tol;
+	c->st_host->maxiter = maxiter;
+	return finish_solve(c, maxiter, final_err, final_iter);
+}
+
 template <bool VIM>
 static int solve_impl(Ctx *c, IMv<VIM> im, int maxiter, double tol, double *final_err, int *final_iter) {
 	const Launch l = launch_shape(c->g);
@@ -664,17 +712,12 @@ static int solve_impl(Ctx *c, IMv<VIM> im, int maxiter, double tol, double *fina
 			return SEDI_ERR_CUDA;
 		}
 	}
-	const SolveState st = *c->st_host;
-	// Entries written: hist[0] plus one per iteration that printed its err
-	// (the s-norm exit and the rho breakdown leave before printing).
-	if (st.reason == STOP_EARLY) c->hist_len = 1;
-	else if (st.reason == STOP_SNORM || st.reason == STOP_RHO) c->hist_len = st.exit_iter;
-	else c->hist_len = (st.exit_iter > maxiter ? maxiter : st.exit_iter) + 1;
-	return finish_result(c, st, final_err, final_iter);
+	return finish_solve(c, maxiter, final_err, final_iter);
 }
 
 // Solve with b, x (and iM when vim) already in the context's buffers.
 int plain_solve_resident(Ctx *c, bool vim, int maxiter, double tol, double *final_err, int *final_iter) {
+	if (!vim && c->res) return resident_solve(c, c->b, c->x, maxiter, tol, final_err, final_iter);
 	if (!vim && c->pairs) {  // n1 even, constant iM: the streaming sweeps
 		const int rc = ensure_hist(c, maxiter);
 		if (rc) return rc;
@@ -692,6 +735,9 @@ int plain_solve_dev(Ctx *c, const double *b, double *x, const double *iM, int ma
                     double *final_err, int *final_iter) {
 	const size_t bytes = sizeof(double) * (size_t)c->g.n;
 	cudaStream_t s = c->stream;
+	// On chip the solve reads b and x once, before it first writes x (b and x may
+	// overlap), and needs no copies of them.
+	if (!iM && c->res) return resident_solve(c, b, x, maxiter, tol, final_err, final_iter);
 	SEDI_TRY(cudaMemcpyAsync(c->b, b, bytes, cudaMemcpyDeviceToDevice, s));
 	SEDI_TRY(cudaMemcpyAsync(c->x, x, bytes, cudaMemcpyDeviceToDevice, s));
 	if (iM) SEDI_TRY(cudaMemcpyAsync(c->iM, iM, bytes, cudaMemcpyDeviceToDevice, s));

@@ -1,0 +1,948 @@
+// Resident solvers: whole Krylov solves in one cooperative launch, with the
+// fields of a right-hand side kept on chip (sm_100a).
+//
+// A grid of up to 148 x 16384 points has Krylov vectors that fit the
+// registers and shared memory of the GPU's 148 SMs.  A group of G blocks (one
+// per SM) then solves one right-hand side (FP64) or two (FP32, a float2 per
+// point): each block owns a box of rows x planes, all n1 points wide, with
+// the stencil input in shared memory (one ghost layer around it) and the
+// residual in registers.  An iteration moves no Krylov vector through HBM; x,
+// which no stencil reads, goes through L2.  CG's two reductions per iteration
+// are the group's only two synchronisations: the one that ends an iteration
+// also publishes the boundary rows of the new residual, from which every
+// block forms its ghost points of the next direction itself.  With more
+// right-hand sides than one group needs blocks for, groups run side by side
+// and take them in turn.
+//
+// Elementwise values round as the sweeps of the other forms: FP64 operator by
+// operator as the reference (Cg.hpp:107-207), FP32 with the products fused
+// into the following sum, so only the dot products' summation order differs.
+#include <cmath>
+#include <cstdio>
+#include <cstring>
+#include <mutex>
+#include <new>
+#include <vector>
+
+#include "resident.cuh"
+#include "sedi_internal.h"
+
+namespace sedi {
+
+// What a launch works on (device pointers; right-hand side k of every field
+// at offset k * npts, or pair k / 2 for float2 fields).
+struct ResArgs {
+	int n1, n2, n3;
+	long long npts;
+	double a, b, c, iM;
+	int lanes;            // right-hand sides
+	int G, groups;        // blocks of a group, groups
+	int s2, RG, nd;       // splits of a group along i2, row groups of a block, planes of a block
+	const double *rhs;    // right-hand sides
+	double *x;            // FP64: x (in: first guess); FP32: x_hi
+	float2 *xlo;          // FP32: correction since the last reliable update
+	void *edge;           // boundary rows of r: [groups][G][2 nd + 2 RG*C][n1] of V
+	Word2 *words;         // [groups][res_words(G)]: the groups' reductions
+	unsigned long long stamp;  // stamps of this launch lie above it
+	double tol, tol_in;   // stop targets (tol_in = theta * tol for FP32)
+	int maxiter, period;
+	double *o_err, *o_bb, *o_rr;  // per right-hand side
+	int *o_exit, *o_reason, *o_done;
+	double *hist;         // err after each iteration of right-hand side 0, or null
+	int *err;             // a wait ran out
+};
+
+namespace {
+
+template <class V>
+struct Lanes;
+template <>
+struct Lanes<double> {
+	typedef double S;
+	static constexpr int N = 1;
+};
+template <>
+struct Lanes<float2> {
+	typedef float S;
+	static constexpr int N = 2;
+};
+__device__ __forceinline__ double lane_get(double v, int) { return v; }
+__device__ __forceinline__ void lane_set(double &v, int, double s) { v = s; }
+__device__ __forceinline__ float lane_get(const float2 &v, int l) { return l ? v.y : v.x; }
+__device__ __forceinline__ void lane_set(float2 &v, int l, float s) {
+	if (l) v.y = s;
+	else v.x = s;
+}
+template <class V>
+__device__ __forceinline__ V lane_zero();
+template <>
+__device__ __forceinline__ double lane_zero<double>() {
+	return 0.0;
+}
+template <>
+__device__ __forceinline__ float2 lane_zero<float2>() {
+	return make_float2(0.f, 0.f);
+}
+
+// r iM + beta p, and x + a y: FP64 rounds each operator, FP32 fuses.
+__device__ __forceinline__ double comb(double r, double im, double beta, double p) {
+	return add(mul(r, im), mul(beta, p));
+}
+__device__ __forceinline__ float comb(float r, float im, float beta, float p) {
+	return __fmaf_rn(r, im, __fmul_rn(beta, p));
+}
+__device__ __forceinline__ double mul_s(double a, double b) { return mul(a, b); }
+__device__ __forceinline__ float mul_s(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double axpy(double x, double a, double y) { return add(x, mul(a, y)); }
+__device__ __forceinline__ float axpy(float x, float a, float y) { return __fmaf_rn(a, y, x); }
+
+// Hides a value's origin, so that the addresses an unrolled loop derives from
+// it are formed there by running increments instead of being kept in (or
+// spilled from) registers across the whole solve.
+__device__ __forceinline__ int opaque(int v) {
+	asm volatile("" : "+r"(v));
+	return v;
+}
+
+// The x an iteration updates: x itself (FP64) or the pair's correction (FP32).
+template <class V>
+__device__ __forceinline__ V *step_x(double *x, float2 *xlo);
+template <>
+__device__ __forceinline__ double *step_x<double>(double *x, float2 *) {
+	return x;
+}
+template <>
+__device__ __forceinline__ float2 *step_x<float2>(double *, float2 *xlo) {
+	return xlo;
+}
+
+// Stencil.hpp:43-50 term order; UNIT: b = c = 1 (exact products left out).
+template <bool UNIT>
+__device__ __forceinline__ double st7r(double a, double b, double c, double xc, double xm1, double xm2, double xm3,
+                                       double xp1, double xp2, double xp3) {
+	double y = mul(a, xc);
+	y = sub(y, UNIT ? xm1 : mul(c, xm1));
+	y = sub(y, UNIT ? xm2 : mul(c, xm2));
+	y = sub(y, UNIT ? xm3 : mul(c, xm3));
+	y = sub(y, UNIT ? xp1 : mul(b, xp1));
+	y = sub(y, UNIT ? xp2 : mul(b, xp2));
+	y = sub(y, UNIT ? xp3 : mul(b, xp3));
+	return y;
+}
+template <bool UNIT>
+__device__ __forceinline__ float st7r(float a, float b, float c, float xc, float xm1, float xm2, float xm3, float xp1,
+                                      float xp2, float xp3) {
+	float y = __fmaf_rn(a, xc, -__fmul_rn(c, xm1));
+	y = __fmaf_rn(-c, xm2, y);
+	y = __fmaf_rn(-c, xm3, y);
+	y = __fmaf_rn(-b, xp1, y);
+	y = __fmaf_rn(-b, xp2, y);
+	y = __fmaf_rn(-b, xp3, y);
+	return y;
+}
+
+// Uniform state of the solve a block runs, in shared memory: written by warp 0
+// at the end of a group sum, read by every thread after it.  Registers are
+// left to the Krylov fields.
+template <int NL>
+struct CgState {
+	const double *rhs[NL];
+	double *x[NL];
+	double bb[NL], rr[NL], ru[NL], alpha[NL], beta[NL], err[NL];
+	double xa[NL];    // step of x still to take, along the p in shared memory
+	int done[NL], reason[NL], ex[NL];
+	int upd[NL];      // FP32: the lane takes part in this iteration's reliable update
+	int restart[NL];  // FP32: p = u after the update
+	int live, any;    // some lane still iterates / is updated
+};
+
+// ---------------------------------------------------------------------------
+// CG.  Block m of a group owns rows [row0, row0 + RG*C) and planes
+// [z0, z0 + nd) of the grid; thread t column i1 = t % n1 of the C consecutive
+// rows of row group t / n1 on every plane, so the stencil marches along i3
+// with the column in registers and takes one i2 neighbour of each of its rows
+// from the row beside it.  Shared memory holds p with its ghosts, rows padded
+// by one zero column that serves both neighbours of the row ends.
+//
+// Per iteration: A: p = u + beta p on the box (where x takes the step along
+// the p that leaves) and, from the published rows of r, on the ghosts; <A p,
+// p>; group sum; B: r -= alpha A p, boundary rows published; <r,u>, <r,r>;
+// group sum.
+//
+// 128^3 FP64: 128 blocks of 128 x 8 x 16 points (186 KB of shared memory, 64
+// registers of r per thread).
+// ---------------------------------------------------------------------------
+template <class V, int C, int D, int TMAX, int BLOCKS, bool UNIT>
+__global__ void __launch_bounds__(TMAX, BLOCKS) k_res_cg(const __grid_constant__ ResArgs A) {
+	typedef typename Lanes<V>::S S;
+	constexpr int NL = Lanes<V>::N;
+	constexpr bool MIXED = NL == 2;
+	constexpr bool KEEP = C * D <= 16;  // A p stays in registers between its two uses
+	extern __shared__ __align__(16) unsigned char smem[];
+	__shared__ ResGroup gsh;
+	__shared__ CgState<NL> st;
+	ResGroup *const g = &gsh;
+	const int t = threadIdx.x, n1 = A.n1;
+	const int B2 = A.RG * C, pitch = n1 + 1, pp = pitch * (B2 + 2);  // box rows, shared row and plane pitches
+	const int i1 = t % n1, rg = t / n1;
+	V *const sp = reinterpret_cast<V *>(smem);
+	const int group = blockIdx.x / A.G;
+	const int s3 = n1 * A.n2;  // the grid has far fewer than 2^31 points
+	int nd, rows, so, go, own3, lo_c, hi_c, lo_d, hi_d;
+	unsigned nbr;  // neighbours: bit 0 i2 low, 1 i2 high, 2 i3 low, 3 i3 high; box rows above
+	{
+		const int m = blockIdx.x % A.G;
+		const int row0 = (m % A.s2) * B2, z0 = (m / A.s2) * A.nd, nr = min(B2, A.n2 - row0);
+		nd = min(A.nd, A.n3 - z0);  // valid planes of the box, nr rows
+		rows = rg < A.RG ? max(0, min(C, nr - rg * C)) : 0;  // valid rows of the thread
+		so = pp + (rg * C + 1) * pitch + 1 + i1;              // own point (c, d) = (0, 0): shared offset
+		go = z0 * s3 + (row0 + rg * C) * n1 + i1;             // and place in the grid
+		own3 = (2 * A.nd + rg * C) * n1 + i1;                 // and in the low i3 face
+		const bool lo2 = row0 > 0, hi2 = row0 + nr < A.n2, lo3 = z0 > 0, hi3 = z0 + nd < A.n3;
+		nbr = (lo2 ? 1u : 0u) | (hi2 ? 2u : 0u) | (lo3 ? 4u : 0u) | (hi3 ? 8u : 0u) | (unsigned)nr << 4;
+		lo_c = lo2 && rg == 0 ? 0 : -1;  // published rows and planes
+		hi_c = hi2 ? nr - 1 - rg * C : -1;
+		lo_d = lo3 ? 0 : -1;
+		hi_d = hi3 ? nd - 1 : -1;
+		if (t == 0) {
+			g->G = A.G;
+			g->m = m;
+			g->words = A.words + (size_t)group * res_words(A.G);
+			g->err = A.err;
+			g->base = A.stamp;
+			g->fail = 0;
+		}
+	}
+	const int face_rows = 2 * A.nd + 2 * B2;  // face rows of a block: i2 low, high, i3 low, high
+	unsigned round = 0;                       // group sums so far
+	V *const faces = static_cast<V *>(A.edge) + (size_t)blockIdx.x * face_rows * n1;  // this block's
+	const S im = (S)A.iM;
+
+	const int units = (A.lanes + NL - 1) / NL;
+	for (int unit = group; unit < units; unit += A.groups) {
+		const int lane0 = unit * NL;
+		if (t == 0)
+			for (int l = 0; l < NL; l++) {
+				const int k = lane0 + l < A.lanes ? lane0 + l : lane0;  // an odd last pair has one right-hand side
+				st.rhs[l] = A.rhs + (size_t)k * A.npts;
+				st.x[l] = A.x + (size_t)k * A.npts;
+			}
+		for (int e = t; e < pp * (A.nd + 2) + 1; e += blockDim.x) sp[e] = lane_zero<V>();
+		__syncthreads();
+		V r[C][D];
+		// The x an iteration updates: x itself (FP64) or the pair's correction.
+		auto step_ptr = [&]() { return step_x<V>(st.x[0], MIXED ? A.xlo + (size_t)unit * A.npts : nullptr); };
+		// r = b - A x from x in global memory (ghost layer zero): the setup and
+		// the FP64 residual of a reliable update.  part: per lane <b,b>, <r,r>,
+		// <r, r iM>; a lane outside the update keeps its r.
+		auto residual = [&](double (&part)[3 * NL], bool setup) {
+#pragma unroll
+			for (int l = 0; l < NL; l++) {
+				part[3 * l] = part[3 * l + 1] = part[3 * l + 2] = 0.0;
+				if (!setup && !st.upd[l]) continue;
+				const double *x = st.x[l], *b = st.rhs[l];
+				const bool live = lane0 + l < A.lanes;
+				const int z0 = go / s3, i2 = (go - z0 * s3) / n1;
+#pragma unroll
+				for (int c = 0; c < C; c++) {
+					int i = opaque(go) + c * n1;
+					const bool ok = c < rows;
+					double prev = (ok && z0 > 0) ? ldl2(x + i - s3) : 0.0, cur = ok ? ldl2(x + i) : 0.0;
+#pragma unroll
+					for (int d = 0; d < D; d++) {
+						if (d < nd && ok) {
+							const double next = z0 + d + 1 < A.n3 ? ldl2(x + i + s3) : 0.0;
+							const double xm1 = i1 > 0 ? ldl2(x + i - 1) : 0.0, xp1 = i1 < n1 - 1 ? ldl2(x + i + 1) : 0.0;
+							const double xm2 = i2 + c > 0 ? ldl2(x + i - n1) : 0.0, xp2 = i2 + c < A.n2 - 1 ? ldl2(x + i + n1) : 0.0;
+							const double ax = st7r<UNIT>(A.a, A.b, A.c, cur, xm1, xm2, prev, xp1, xp2, next);
+							const double bi = live ? b[i] : 0.0;
+							const double ri = live ? add(bi, -ax) : 0.0;  // combine2(1.0, b, -1.0, A x) (Cg.hpp:123)
+							const S rt = (S)ri;
+							lane_set(r[c][d], l, rt);
+							part[3 * l] = fma(bi, bi, part[3 * l]);
+							part[3 * l + 1] = fma(ri, ri, part[3 * l + 1]);
+							if (setup) part[3 * l + 2] = fma((double)rt, (double)mul_s(rt, im), part[3 * l + 2]);
+							else part[3 * l + 2] = fma(ri, mul(ri, A.iM), part[3 * l + 2]);
+							prev = cur;
+							cur = next;
+							i += s3;
+							asm volatile("" ::: "memory");  // one point's loads at a time: registers hold r
+						} else if (setup) {
+							lane_set(r[c][d], l, (S)0);
+						}
+					}
+				}
+			}
+		};
+		// Publishes a point of the box's faces (f2, f3: the thread's place in the
+		// i2 and i3 faces) for the neighbours to read after the next fenced sum.
+		auto publish = [&](int c, int d, int f2, int f3, const V &v) {
+			if (c == lo_c) stl2(faces + f2, v);
+			if (c == hi_c) stl2(faces + f2 + A.nd * n1, v);
+			if (d == lo_d) stl2(faces + f3 + c * n1, v);
+			if (d == hi_d) stl2(faces + f3 + (B2 + c) * n1, v);
+		};
+		auto publish_all = [&]() {
+			int f2 = opaque(i1);
+			const int f3 = opaque(own3);
+#pragma unroll
+			for (int d = 0; d < D; d++, f2 += n1)
+#pragma unroll
+				for (int c = 0; c < C; c++)
+					if (c < rows && d < nd) publish(c, d, f2, f3, r[c][d]);
+		};
+
+		{
+			double part[3 * NL];
+			residual(part, true);
+			publish_all();
+			if (!group_sum<3 * NL, true>(g, round, part, Nothing(), [&](int lane, const double (&v)[3 * NL]) {
+				    if (lane == 0) {
+					    int live = 0;
+#pragma unroll
+					    for (int l = 0; l < NL; l++) {
+						    const double bb = v[3 * l] == 0.0 ? 1.0 : v[3 * l];  // Cg.hpp:112-115
+						    const double err = sqrt(__ddiv_rn(v[3 * l + 1], bb));
+						    int done = 0, reason = STOP_NONE, ex = 0;
+						    if (lane0 + l >= A.lanes) {
+							    done = 1;
+						    } else if (err < A.tol) {  // :130-134
+							    done = 1;
+							    reason = STOP_EARLY;
+						    } else if (A.maxiter < 1) {
+							    done = 1;
+							    reason = STOP_MAXITER;
+							    ex = 1;
+						    }
+						    st.bb[l] = bb;
+						    st.rr[l] = v[3 * l + 1];
+						    st.ru[l] = v[3 * l + 2];
+						    st.err[l] = err;
+						    st.beta[l] = st.xa[l] = 0.0;
+						    st.done[l] = done;
+						    st.reason[l] = reason;
+						    st.ex[l] = ex;
+						    st.upd[l] = st.restart[l] = 0;
+						    live |= !done;
+					    }
+					    st.live = live;
+					    if (A.hist && unit == 0 && blockIdx.x % A.G == 0) A.hist[0] = st.err[0];
+				    }
+			    }))
+				return;
+		}
+		if (MIXED) {
+			V *xs = step_ptr() + go;
+			for (int d = 0; d < nd; d++, xs += s3)
+#pragma unroll
+				for (int c = 0; c < C; c++)
+					if (c < rows) stl2(xs + c * n1, lane_zero<V>());
+		}
+
+		for (int it = 1; st.live; it++) {
+			// ---- A: p = u + beta p (Cg.hpp:188) on the ghosts, from the neighbours' r, and on the box.
+			if (rg < A.RG) {
+				S be[NL];
+#pragma unroll
+				for (int l = 0; l < NL; l++) be[l] = (S)st.beta[l];
+				// Ghost rows: nd on each i2 side, nr on each i3 side, dealt to the row groups.
+				const int nr = (int)(nbr >> 4), ghosts = 2 * nd + 2 * nr;
+				constexpr int HB = 6;
+				for (int h0 = rg; h0 < ghosts; h0 += HB * A.RG) {
+					V rh[HB];
+					int off[HB];
+#pragma unroll
+					for (int k = 0; k < HB; k++) {
+						const int h = h0 + k * A.RG;
+						off[k] = -1;
+						if (h >= ghosts) continue;
+						// Ghost row h: box row j2 and plane j3 (-1 and nr / nd outside the
+						// box), the face row of the neighbour it comes from.
+						int j2, j3, fr;
+						unsigned side;
+						if (h < 2 * nd) {
+							const bool hi = h >= nd;
+							j3 = hi ? h - nd : h;
+							j2 = hi ? nr : -1;
+							side = hi ? 2u : 1u;
+							fr = hi ? face_rows + j3 : -face_rows + A.nd + j3;
+						} else {
+							const bool hi = h >= 2 * nd + nr;
+							j2 = hi ? h - 2 * nd - nr : h - 2 * nd;
+							j3 = hi ? nd : -1;
+							side = hi ? 8u : 4u;
+							fr = 2 * A.nd + j2 + (hi ? A.s2 * face_rows : B2 - A.s2 * face_rows);
+						}
+						if (!(nbr & side)) continue;
+						off[k] = (j3 + 1) * pp + (j2 + 1) * pitch + 1 + i1;
+						rh[k] = ldl2(faces + fr * n1 + i1);
+					}
+#pragma unroll
+					for (int k = 0; k < HB; k++) {
+						if (off[k] < 0) continue;
+						V p = sp[off[k]];
+#pragma unroll
+						for (int l = 0; l < NL; l++) lane_set(p, l, comb(lane_get(rh[k], l), im, be[l], lane_get(p, l)));
+						sp[off[k]] = p;
+					}
+				}
+				// x takes the step of the iteration before here, where its p is read
+				// anyway; x of the next plane is on its way, and the stores drain
+				// during the stencil.
+				S ax[NL];
+				bool step = false;
+#pragma unroll
+				for (int l = 0; l < NL; l++) {
+					ax[l] = (S)st.xa[l];
+					step |= st.xa[l] != 0.0;
+				}
+				V *xp = step_ptr() + opaque(go);
+				V *q = sp + opaque(so);
+				V xn[C];
+				auto load_x = [&](int d) {
+					if (step && d < nd)
+#pragma unroll
+						for (int c = 0; c < C; c++)
+							if (c < rows) xn[c] = ldl2(xp + c * n1);
+				};
+				load_x(0);
+#pragma unroll
+				for (int d = 0; d < D; d++, q += pp) {
+					if (d >= nd) break;
+					V x[C];
+#pragma unroll
+					for (int c = 0; c < C; c++) x[c] = xn[c];
+					xp += s3;
+					load_x(d + 1);
+#pragma unroll
+					for (int c = 0; c < C; c++) {
+						if (c >= rows) continue;
+						V p = q[c * pitch];
+						if (step) {
+#pragma unroll
+							for (int l = 0; l < NL; l++)
+								if (NL == 1 || ax[l] != (S)0) lane_set(x[c], l, axpy(lane_get(x[c], l), ax[l], lane_get(p, l)));
+							stl2(xp - s3 + c * n1, x[c]);
+						}
+#pragma unroll
+						for (int l = 0; l < NL; l++)
+							lane_set(p, l, comb(lane_get(r[c][d], l), im, be[l], lane_get(p, l)));
+						q[c * pitch] = p;
+					}
+				}
+			}
+			__syncthreads();
+			// Stencil march over the thread's rows: f(c, d, p, A p) of its points.
+			auto march_rows = [&](auto f) {
+				const S ka = (S)A.a, kb = (S)A.b, kc = (S)A.c;
+				const V *q = sp + opaque(so);
+				V prev[C], cur[C];
+#pragma unroll
+				for (int c = 0; c < C; c++) {
+					prev[c] = q[c * pitch - pp];
+					cur[c] = q[c * pitch];
+				}
+#pragma unroll
+				for (int d = 0; d < D; d++) {
+					if (d >= nd) break;
+					V next[C];
+#pragma unroll
+					for (int c = 0; c < C; c++) next[c] = q[pp + c * pitch];
+					const V up = q[-pitch], dn = q[C * pitch];
+#pragma unroll
+					for (int c = 0; c < C; c++) {
+						const V xm1 = q[c * pitch - 1], xp1 = q[c * pitch + 1];
+						const V &xm2 = c > 0 ? cur[c > 0 ? c - 1 : 0] : up;
+						const V &xp2 = c + 1 < C ? cur[c + 1 < C ? c + 1 : c] : dn;
+						V y;
+#pragma unroll
+						for (int l = 0; l < NL; l++)
+							lane_set(y, l, st7r<UNIT>(ka, kb, kc, lane_get(cur[c], l), lane_get(xm1, l), lane_get(xm2, l),
+							                          lane_get(prev[c], l), lane_get(xp1, l), lane_get(xp2, l),
+							                          lane_get(next[c], l)));
+						f(c, d, cur[c], y);
+					}
+#pragma unroll
+					for (int c = 0; c < C; c++) {
+						prev[c] = cur[c];
+						cur[c] = next[c];
+					}
+					q += pp;
+				}
+			};
+			V ap[C][KEEP ? D : 1];
+			{
+				double v[NL];
+#pragma unroll
+				for (int l = 0; l < NL; l++) v[l] = 0.0;
+				if (rows > 0)
+					march_rows([&](int c, int d, const V &p, const V &s) {
+						if (KEEP) ap[c][KEEP ? d : 0] = s;
+						if (c < rows)
+#pragma unroll
+							for (int l = 0; l < NL; l++) v[l] = fma((double)lane_get(s, l), (double)lane_get(p, l), v[l]);
+					});
+				if (!group_sum<NL>(g, round, v, Nothing(), [&](int lane, const double (&tot)[NL]) {
+#pragma unroll
+					    for (int l = 0; l < NL; l++)
+						    if (lane == l) {
+							    double a = __ddiv_rn(st.ru[l], tot[l]);  // :166
+							    st.upd[l] = 0;
+							    if (st.done[l]) {
+								    a = 0.0;
+							    } else if (MIXED && !(tot[l] > 0.0 && isfinite(a))) {
+								    // FP32 breakdown (p = 0 once the recurrence residual is exactly
+								    // zero, or overflow): no step, then a restart from the true residual.
+								    a = 0.0;
+								    st.upd[l] = st.restart[l] = 1;
+							    }
+							    st.alpha[l] = st.xa[l] = a;
+						    }
+				    }))
+					return;
+			}
+			const bool periodic = MIXED && A.period > 0 && it % A.period == 0;
+			// ---- B: r -= alpha s, u = r iM (:172-175); the boundary rows of r go out.
+			{
+				double v[2 * NL];
+#pragma unroll
+				for (int d = 0; d < 2 * NL; d++) v[d] = 0.0;
+				if (rows > 0) {
+					S al[NL];
+#pragma unroll
+					for (int l = 0; l < NL; l++) al[l] = -(S)st.alpha[l];
+					int f2 = opaque(i1);
+					const int f3 = opaque(own3);
+					auto update = [&](int c, int d, const V &, const V &s) {
+						if (c < rows) {
+							V rv = r[c][d];
+#pragma unroll
+							for (int l = 0; l < NL; l++) {
+								const S q = axpy(lane_get(rv, l), al[l], lane_get(s, l));
+								lane_set(rv, l, q);
+								v[2 * l] = fma((double)q, (double)mul_s(q, im), v[2 * l]);
+								v[2 * l + 1] = fma((double)q, (double)q, v[2 * l + 1]);
+							}
+							r[c][d] = rv;
+							publish(c, d, f2, f3, rv);
+						}
+						if (c == C - 1) f2 += n1;
+					};
+					if (KEEP) {
+#pragma unroll
+						for (int d = 0; d < D; d++) {
+							if (d >= nd) break;
+#pragma unroll
+							for (int c = 0; c < C; c++) update(c, d, ap[c][KEEP ? d : 0], ap[c][KEEP ? d : 0]);
+						}
+					} else {
+						march_rows(update);
+					}
+				}
+				if (!group_sum<2 * NL, true>(g, round, v, Nothing(), [&](int lane, const double (&tot)[2 * NL]) {
+#pragma unroll
+					    for (int l = 0; l < NL; l++) {
+						    // Lane 2l: beta; lane 2l + 1: the error and the stop test.
+						    if (lane / 2 != l || st.done[l]) continue;
+						    const bool e = lane & 1;
+						    const double q = __ddiv_rn(e ? tot[2 * l + 1] : tot[2 * l], e ? st.bb[l] : st.ru[l]);
+						    if (!e) {
+							    st.beta[l] = q;  // :185
+							    continue;
+						    }
+						    const double err = sqrt(q);  // :191
+						    st.rr[l] = tot[2 * l + 1];
+						    st.err[l] = err;
+						    if (A.hist && unit == 0 && l == 0 && blockIdx.x % A.G == 0) A.hist[it] = err;
+						    if (MIXED) {
+							    // The FP32 recurrence only proposes; the FP64 true residual decides.
+							    if (!(err == err)) st.restart[l] = 1;
+							    if (err <= A.tol_in || it >= A.maxiter || !(err == err) || periodic) st.upd[l] = 1;
+						    } else if (err <= A.tol_in) {  // :193
+							    st.done[l] = 1;
+							    st.ex[l] = it;
+							    st.reason[l] = STOP_CONVERGED;
+						    } else if (it >= A.maxiter) {
+							    st.done[l] = 1;
+							    st.ex[l] = A.maxiter + 1;
+							    st.reason[l] = STOP_MAXITER;
+						    }
+					    }
+					    __syncwarp();
+					    if (lane == 0) {
+						    st.live = st.any = 0;
+#pragma unroll
+						    for (int l = 0; l < NL; l++) {
+							    st.live |= !st.done[l];
+							    st.any |= !st.done[l] && st.upd[l];
+							    if (st.done[l]) st.beta[l] = 0.0;
+							    // An update forms its beta over the old <r,u> first.
+							    if (!MIXED || !st.upd[l]) st.ru[l] = tot[2 * l];
+						    }
+					    }
+				    }))
+					return;
+			}
+			if (MIXED && st.any) {
+				// Reliable update: x_hi += x_lo and the pending step (in FP32 through
+				// x_lo after an even iteration, in FP64 after an odd one and then only
+				// for lanes in the update), then r = b - A x_hi in FP64.  Both lanes of
+				// a pair fold their x_lo; only lanes in the update take a new r.
+				const bool odd = it & 1;
+				{
+					V *xp = step_ptr() + go;
+					int i = go;
+					const V *q = sp + so;
+					for (int d = 0; d < nd; d++, i += s3, xp += s3, q += pp)
+#pragma unroll
+						for (int c = 0; c < C; c++) {
+							if (c >= rows) continue;
+							const V p = q[c * pitch], x = ldl2(xp + c * n1);
+#pragma unroll
+							for (int l = 0; l < NL; l++) {
+								if (lane0 + l >= A.lanes) continue;
+								double *const xh = st.x[l] + i + c * n1;
+								S lo = lane_get(x, l);
+								if (!odd && st.xa[l] != 0.0) lo = axpy(lo, (S)st.xa[l], lane_get(p, l));
+								double hi = ldl2(xh) + (double)lo;
+								if (odd && st.upd[l] && !st.done[l]) hi = fma(st.xa[l], (double)lane_get(p, l), hi);
+								stl2(xh, hi);
+							}
+							stl2(xp + c * n1, lane_zero<V>());
+						}
+				}
+				double part[3 * NL];
+				part[0] = 0.0;
+				double none[1] = {0.0};
+				if (!group_sum<1, true>(g, round, none, Nothing(), [&](int lane, const double (&)[1]) {
+					    if (lane < NL && (!odd || (st.upd[lane] && !st.done[lane]))) st.xa[lane] = 0.0;
+				    }))
+					return;  // x_hi complete
+				residual(part, false);
+				publish_all();
+				if (!group_sum<3 * NL, true>(g, round, part, Nothing(), [&](int lane, const double (&tot)[3 * NL]) {
+					    if (lane != 0) return;
+					    st.live = 0;
+#pragma unroll
+					    for (int l = 0; l < NL; l++) {
+						    if (!st.done[l] && st.upd[l]) {
+							    const double rr = tot[3 * l + 1], ru = tot[3 * l + 2];
+							    // A recurrence residual far below the true one (squared norms 1e-6
+							    // apart) no longer describes it: restart from the replaced one.
+							    const bool lost = !(st.rr[l] >= 1e-6 * rr);
+							    const double err = sqrt(rr / st.bb[l]);
+							    st.rr[l] = rr;
+							    st.err[l] = err;
+							    if (err <= A.tol_in) {
+								    st.done[l] = 1;
+								    st.ex[l] = it;
+								    st.reason[l] = STOP_CONVERGED;
+							    } else if (it >= A.maxiter) {
+								    st.done[l] = 1;
+								    st.ex[l] = A.maxiter + 1;
+								    st.reason[l] = STOP_MAXITER;
+							    } else {
+								    double be = ru / st.ru[l];
+								    if (lost || st.restart[l] || !(be >= 0.0 && isfinite(be))) be = 0.0;  // p = u
+								    st.beta[l] = be;
+								    st.ru[l] = ru;
+								    st.restart[l] = 0;
+							    }
+							    if (st.done[l]) st.beta[l] = 0.0;
+						    }
+						    st.live |= !st.done[l];
+					    }
+				    }))
+					return;
+			}
+		}
+		if (!MIXED && st.xa[0] != 0.0) {  // the last iteration's step (FP32: x_hi is complete)
+			V *xp = step_ptr() + go;
+			const V *q = sp + so;
+			for (int d = 0; d < nd; d++, xp += s3, q += pp)
+#pragma unroll
+				for (int c = 0; c < C; c++) {
+					if (c >= rows) continue;
+					V x = ldl2(xp + c * n1);
+					lane_set(x, 0, axpy(lane_get(x, 0), (S)st.xa[0], lane_get(q[c * pitch], 0)));
+					stl2(xp + c * n1, x);
+				}
+		}
+		if (blockIdx.x % A.G == 0 && t == 0)
+			for (int l = 0; l < NL; l++) {
+				const int k = lane0 + l;
+				if (k >= A.lanes) continue;
+				A.o_err[k] = st.err[l];
+				A.o_bb[k] = st.bb[l];
+				A.o_rr[k] = st.rr[l];
+				A.o_exit[k] = st.ex[l];
+				A.o_reason[k] = st.reason[l];
+				A.o_done[k] = 1;
+			}
+		__syncthreads();  // shared memory is reused by the next right-hand side
+	}
+}
+
+}  // namespace
+
+// ---------------------------------------------------------------------------
+// Host side.
+// ---------------------------------------------------------------------------
+namespace {
+
+typedef void (*ResKernel)(const ResArgs);
+
+// Box shapes: C rows x at most D planes per thread, at most T threads, so many
+// blocks per SM.
+constexpr int kShapes = 6;
+constexpr int kShapeC[kShapes] = {1, 1, 2, 2, 3, 2}, kShapeD[kShapes] = {2, 8, 8, 16, 16, 16},
+              kShapeT[kShapes] = {512, 512, 512, 512, 384, 256}, kShapeB[kShapes] = {1, 1, 1, 1, 1, 2};
+
+template <class V, bool UNIT>
+ResKernel cg_kernel(int shape) {
+	switch (shape) {
+	case 0: return k_res_cg<V, 1, 2, 512, 1, UNIT>;
+	case 1: return k_res_cg<V, 1, 8, 512, 1, UNIT>;
+	case 2: return k_res_cg<V, 2, 8, 512, 1, UNIT>;
+	case 3: return k_res_cg<V, 2, 16, 512, 1, UNIT>;
+	case 4: return k_res_cg<V, 3, 16, 384, 1, UNIT>;
+	default: return k_res_cg<V, 2, 16, 256, 2, UNIT>;
+	}
+}
+
+ResKernel kernel_for(bool fp32, bool unit, int shape) {
+	if (fp32) return cg_kernel<float2, false>(shape);  // FP32 folds b, c into its multiply-adds
+	return unit ? cg_kernel<double, true>(shape) : cg_kernel<double, false>(shape);
+}
+
+struct Plan {
+	int shape = -1, G = 0, groups = 0, RG = 0, T = 0, s2 = 0, nd = 0;
+	size_t smem = 0;
+};
+
+// Plan with the smallest estimated time of an iteration of `units` solves, and
+// that time in cycles.  Measured on B200 (FP64, 1.95 GHz): the two reductions,
+// ghost rows and launch of each phase take 9000-11000 cycles between blocks;
+// a point adds 1.3 where A p stays in registers (2048 points a block 13600, 8192
+// 20100), 1.65 with two stencil passes (16384: 38000), 1.8 at three rows a
+// thread (12672: 32500), and 3.2 with two blocks on an SM (2 x 8192: 37400).
+Plan plan_for(const Geo &g, int units, int sms, size_t smem_max, double *cycles) {
+	constexpr double kPoint[kShapes] = {1.3, 1.3, 1.3, 1.65, 1.8, 3.2};
+	Plan best;
+	for (int sh = 0; sh < kShapes; sh++) {
+		const int C = kShapeC[sh], slots = sms * kShapeB[sh];  // blocks at once
+		for (int RG = kShapeT[sh] / g.n1; RG >= 1; RG--) {
+			if (RG > 1 && (RG - 1) * C >= g.n2) continue;  // a row group with nothing to do
+			const int T = (RG * g.n1 + 31) / 32 * 32, B2 = RG * C, s2 = (g.n2 + B2 - 1) / B2;
+			for (int nd = 1; nd <= kShapeD[sh] && nd <= g.n3; nd++) {
+				const long long G = (long long)s2 * ((g.n3 + nd - 1) / nd);
+				const size_t smem = ((size_t)(g.n1 + 1) * (B2 + 2) * (nd + 2) + 1) * 8;
+				if (G > slots || smem * kShapeB[sh] > smem_max) continue;
+				const int groups = units < slots / (int)G ? units : slots / (int)G;
+				const double cost = ((G > 1 ? 9000.0 + 15.0 * G : 3000.0) + kPoint[sh] * T * C * nd) *
+				                    ((units + groups - 1) / groups);
+				if (best.shape >= 0 && cost >= *cycles) continue;
+				*cycles = cost;
+				best.shape = sh;
+				best.G = (int)G;
+				best.groups = groups;
+				best.RG = RG;
+				best.T = T;
+				best.s2 = s2;
+				best.nd = nd;
+				best.smem = smem;
+			}
+		}
+	}
+	return best;
+}
+
+// Estimated time of an iteration of the streaming sweeps on a batch, in cycles
+// of the same clock: launches and latency, then HBM (CG: 7.5 words per point
+// and lane), more where the tiles overhang the grid.  Measured (us): FP64
+// 32^3 x 16 27, 64^3 x 64 188, 96^3 x 64 578, 128^3 x 64 1418; FP32 64^3 x 64
+// 122, 96^3 x 64 320, 128^3 x 64 798.
+double stream_cycles(const Geo &g, int lanes, bool fp32) {
+	const double over = (double)((g.n1 + 31) / 32 * 32) * ((g.n2 + 31) / 32 * 32) / ((double)g.n1 * g.n2);
+	return 1950.0 * (26.0 + 7.5 * (fp32 ? 4.0 : 8.0) * (double)g.n * lanes * std::sqrt(over) / 5.9e6);
+}
+
+size_t word_bytes(const Plan &p) { return sizeof(Word2) * res_words(p.G) * p.groups; }
+
+size_t edge_bytes(const Plan &p, const Geo &g) {
+	return 8 * (size_t)p.groups * p.G * (2 * p.nd + 2 * p.RG * kShapeC[p.shape]) * g.n1;
+}
+
+}  // namespace
+
+struct Resident {
+	Plan plan;
+	bool fp32 = false, unit = false;
+	Word2 *words = nullptr;
+	void *edge = nullptr;
+	unsigned long long launch = 0;
+	int device = 0, sms = 0;
+	cudaEvent_t done = nullptr;  // after the latest launch
+	int held = 0;                // SMs of that launch while it may run
+};
+
+// Launches that may be running, oldest first.  The blocks of a launch wait for
+// one another, so all of them must find room: two launches that each hold a
+// part of the GPU and wait for the rest would never end.  A new launch
+// therefore waits (on its stream) for the oldest ones until those it may
+// overlap and itself need no more SMs than there are.  Other kernels end by
+// themselves.  One entry per context, taken out when the context goes.
+static std::mutex g_running_mu;
+static std::vector<Resident *> g_running;
+
+static void running_remove(Resident *R) {
+	for (size_t i = 0; i < g_running.size(); i++)
+		if (g_running[i] == R) {
+			g_running.erase(g_running.begin() + (long)i);
+			return;
+		}
+}
+
+// A resident solver for `lanes` right-hand sides of the context's grid; *out
+// stays null where the grid or the device does not take one (the streaming
+// and march kernels serve those).
+int resident_alloc(Ctx *c, int ks, bool fp32, int lanes, Resident **out) {
+	*out = nullptr;
+	if (ks != SEDI_CG) return 0;
+	if (c->g.n1 > 512 || c->g.n > (1 << 22)) return 0;  // no box shape takes them
+	int sms = 0, coop = 0, smem_max = 0;
+	const bool unit = c->k.b == 1.0 && c->k.c == 1.0;
+	if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device) != cudaSuccess ||
+	    cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, c->device) != cudaSuccess ||
+	    cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device) != cudaSuccess || !coop) {
+		cudaGetLastError();
+		return 0;
+	}
+	// Beside the static arrays and what the system keeps, for up to two blocks of an SM.
+	const size_t shared = (size_t)smem_max - 2 * (sizeof(ResGroup) + sizeof(CgState<2>) + 1024);
+	if (sms > kResMaxBlocks / 2) sms = kResMaxBlocks / 2;
+	double cycles = 0.0;
+	const Plan p = plan_for(c->g, fp32 ? (lanes + 1) / 2 : lanes, sms, shared, &cycles);
+	if (p.shape < 0) return 0;
+	// A pair of FP32 lanes takes 1.6-1.9 times an FP64 lane (conversions for its
+	// FP64 sums).  One right-hand side has no streaming form at these sizes
+	// (its march kernels take 12 us an iteration at 32^3, 47 at 128^3; this 5.6
+	// and 20), a batch does.
+	if (fp32) cycles *= 1.8;
+	if (lanes > 1 && cycles > stream_cycles(c->g, lanes, fp32)) return 0;
+	const ResKernel k = kernel_for(fp32, unit, p.shape);
+	int per_sm = 0;
+	// (The attribute is the kernel's, whoever launches it: its largest use.)
+	if (cudaFuncSetAttribute((const void *)k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+	                         (int)(shared / kShapeB[p.shape])) != cudaSuccess ||
+	    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void *)k, p.T, p.smem) != cudaSuccess || per_sm < kShapeB[p.shape]) {
+		cudaGetLastError();
+		return 0;
+	}
+	Resident *R = new (std::nothrow) Resident();
+	if (!R) return SEDI_ERR_NOMEM;
+	R->plan = p;
+	R->fp32 = fp32;
+	R->unit = unit;
+	R->device = c->device;
+	R->sms = sms;
+	if (cudaMalloc(&R->words, word_bytes(p)) != cudaSuccess || cudaMalloc(&R->edge, edge_bytes(p, c->g)) != cudaSuccess ||
+	    cudaEventCreateWithFlags(&R->done, cudaEventDisableTiming) != cudaSuccess) {
+		cudaGetLastError();
+		resident_free(R);
+		c->error = "device allocation failed (resident solver)";
+		return SEDI_ERR_NOMEM;
+	}
+	// No word may carry a stamp of a launch to come.
+	cudaMemsetAsync(R->words, 0, word_bytes(p), c->stream);
+	cudaMemsetAsync(R->edge, 0, edge_bytes(p, c->g), c->stream);
+	*out = R;
+	return cudaStreamSynchronize(c->stream) == cudaSuccess ? 0 : set_cuda_error(c, cudaGetLastError(), "resident_alloc");
+}
+
+void resident_free(Resident *R) {
+	if (!R) return;
+	{
+		std::lock_guard<std::mutex> lk(g_running_mu);
+		running_remove(R);
+	}
+	if (R->done) cudaEventDestroy(R->done);
+	if (R->words) cudaFree(R->words);
+	if (R->edge) cudaFree(R->edge);
+	delete R;
+}
+
+// Solves io.lanes right-hand sides on the context's stream.
+int resident_launch(Ctx *c, Resident *R, const ResIO &io) {
+	const Plan &p = R->plan;
+	const int units = R->fp32 ? (io.lanes + 1) / 2 : io.lanes, groups = units < p.groups ? units : p.groups;
+	if (units < 1) return 0;
+	ResArgs a;
+	a.n1 = c->g.n1;
+	a.n2 = c->g.n2;
+	a.n3 = c->g.n3;
+	a.npts = c->g.n;
+	a.a = c->k.a;
+	a.b = c->k.b;
+	a.c = c->k.c;
+	a.iM = 1.0 / c->k.a;  // stochastic-estimator.cc:103
+	a.lanes = io.lanes;
+	a.G = p.G;
+	a.groups = groups;
+	a.s2 = p.s2;
+	a.RG = p.RG;
+	a.nd = p.nd;
+	a.rhs = io.rhs;
+	a.x = io.x;
+	a.xlo = (float2 *)io.xlo;
+	a.edge = R->edge;
+	a.words = R->words;
+	a.stamp = ++R->launch << 36;
+	a.tol = io.tol;
+	a.tol_in = io.tol_in;
+	a.maxiter = io.maxiter;
+	a.period = io.period;
+	a.o_err = io.o_err;
+	a.o_bb = io.o_bb;
+	a.o_rr = io.o_rr;
+	a.o_exit = io.o_exit;
+	a.o_reason = io.o_reason;
+	a.o_done = io.o_done;
+	a.hist = io.hist;
+	a.err = io.err;
+	void *args[] = {&a};
+	const int blocks = groups * p.G, per_sm = kShapeB[p.shape], need = p.G > 1 ? (blocks + per_sm - 1) / per_sm : 0;
+	std::lock_guard<std::mutex> lk(g_running_mu);
+	running_remove(R);
+	int held = need;
+	for (size_t i = 0; i < g_running.size();) {
+		Resident *const o = g_running[i];
+		if (o->device == R->device) {
+			if (cudaEventQuery(o->done) == cudaSuccess) {
+				g_running.erase(g_running.begin() + (long)i);
+				continue;
+			}
+			held += o->held;
+		}
+		i++;
+	}
+	for (size_t i = 0; need > 0 && held > R->sms && i < g_running.size(); i++) {
+		Resident *const o = g_running[i];
+		if (o->device != R->device) continue;
+		const cudaError_t w = cudaStreamWaitEvent(c->stream, o->done, 0);
+		if (w != cudaSuccess) return set_cuda_error(c, w, "resident solver launch");
+		held -= o->held;
+	}
+	cudaError_t e = cudaLaunchCooperativeKernel((const void *)kernel_for(R->fp32, R->unit, p.shape), dim3((unsigned)blocks),
+	                                            dim3((unsigned)p.T), args, p.smem, c->stream);
+	if (e == cudaSuccess && need > 0) {
+		e = cudaEventRecord(R->done, c->stream);
+		R->held = need;
+		g_running.push_back(R);
+	}
+	if (e != cudaSuccess) return set_cuda_error(c, e, "resident solver launch");
+	c->launches++;
+	return 0;
+}
+
+}  // namespace sedi

@@ -47,8 +47,10 @@ struct SolveState {
 	// BiCGStab
 	double rho, rho_prev, omega, vr, s_norm2, ts, tt;
 	int s_exit;
-	int pad1;
+	int wait_err;    // a resident solve's wait ran out
 };
+
+struct Resident;  // resident.cu
 
 struct Ctx {
 	int solver, precision, batch, mode;
@@ -78,6 +80,7 @@ struct Ctx {
 	size_t stage_probe_bytes;
 
 	void *batched;  // batched-form state (batched.cu)
+	Resident *res;  // single-vector form with the whole solve on chip (grids that fit), or null
 	void *pairs;    // single-vector form on the streaming sweeps (n1 even; batched.cu)
 
 	long long launches;
@@ -139,6 +142,23 @@ double batched_theta(const Ctx *c);
 size_t batched_bytes(int solver, int precision, int batch, long long n1, long long n2, long long n3);
 // Lanes (padded right-hand sides) of a batched context created for `batch`.
 int batched_lanes(int precision, int batch);
+
+// resident.cu: whole solves in one launch, Krylov fields on chip.
+struct ResIO {
+	int lanes;             // right-hand sides, dense: vector k at offset k * n
+	const double *rhs;
+	double *x;             // FP64: x; FP32: x_hi
+	void *xlo;             // FP32: scratch of one Krylov field
+	double tol, tol_in;
+	int maxiter, period;
+	double *o_err, *o_bb, *o_rr;  // device, per right-hand side
+	int *o_exit, *o_reason, *o_done;
+	double *hist;
+	int *err;
+};
+int resident_alloc(Ctx *c, int ks, bool fp32, int lanes, Resident **out);
+void resident_free(Resident *R);
+int resident_launch(Ctx *c, Resident *R, const ResIO &io);
 
 // rng.cu
 void host_fill_probe(uint32_t seed, long n, double *out);
