@@ -2393,6 +2393,11 @@ static int resident_chunk(Ctx *c, Batched *B) {
 	io.o_exit = B->ls.exit_iter;
 	io.o_reason = B->ls.reason;
 	io.o_done = B->ls.done;
+	if (B->ks == SEDI_BICGSTAB) {
+		io.o_snorm = B->ls.s_norm2;
+		io.o_omega = B->ls.omega;
+		io.o_rho = B->ls.rho;
+	}
 	io.err = &B->gl->err;
 	return resident_launch(c, B->res, io);
 }

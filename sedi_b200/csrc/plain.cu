@@ -665,6 +665,11 @@ static int resident_solve(Ctx *c, const double *b, double *x, int maxiter, doubl
 	io.o_exit = &c->st->exit_iter;
 	io.o_reason = &c->st->reason;
 	io.o_done = &c->st->done;
+	if (c->solver == SEDI_BICGSTAB) {
+		io.o_snorm = &c->st->s_norm2;
+		io.o_omega = &c->st->omega;
+		io.o_rho = &c->st->rho;
+	}
 	io.hist = c->hist;
 	io.err = &c->st->wait_err;
 	const int e = resident_launch(c, c->res, io);

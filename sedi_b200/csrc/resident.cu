@@ -41,13 +41,14 @@ struct ResArgs {
 	const double *rhs;    // right-hand sides
 	double *x;            // FP64: x (in: first guess); FP32: x_hi
 	float2 *xlo;          // FP32: correction since the last reliable update
-	void *edge;           // boundary rows of r: [groups][G][2 nd + 2 RG*C][n1] of V
+	void *edge;           // boundary rows: [fields][groups][G][2 nd + 2 RG*C][n1] of V
 	Word2 *words;         // [groups][res_words(G)]: the groups' reductions
 	unsigned long long stamp;  // stamps of this launch lie above it
 	double tol, tol_in;   // stop targets (tol_in = theta * tol for FP32)
 	int maxiter, period;
 	double *o_err, *o_bb, *o_rr;  // per right-hand side
 	int *o_exit, *o_reason, *o_done;
+	double *o_snorm, *o_omega, *o_rho;  // BiCGStab, else null
 	double *hist;         // err after each iteration of right-hand side 0, or null
 	int *err;             // a wait ran out
 };
@@ -683,6 +684,479 @@ __global__ void __launch_bounds__(TMAX, BLOCKS) k_res_cg(const __grid_constant__
 	}
 }
 
+// ---------------------------------------------------------------------------
+// A block's box and a thread's column in it, for solvers whose stencil input
+// is in shared memory with its ghosts (one row per thread and plane).
+// ---------------------------------------------------------------------------
+struct ResBox {
+	int i1, rg, pitch, pp;    // column, row group (= box row); shared row and plane pitches
+	int nd, nr;               // valid planes and rows of the box
+	int so, go, s3;           // own point of plane 0: shared offset, place in the grid; plane stride
+	int z0, row0, face_rows;
+	bool own, lo2, hi2, lo3, hi3;
+	__device__ ResBox(const ResArgs &A) {
+		const int m = blockIdx.x % A.G, n1 = A.n1;
+		i1 = threadIdx.x % n1;
+		rg = threadIdx.x / n1;
+		pitch = n1 + 1;
+		pp = pitch * (A.RG + 2);
+		row0 = (m % A.s2) * A.RG;
+		z0 = (m / A.s2) * A.nd;
+		nr = min(A.RG, A.n2 - row0);
+		nd = min(A.nd, A.n3 - z0);
+		own = rg < nr;
+		s3 = n1 * A.n2;
+		so = pp + (rg + 1) * pitch + 1 + i1;
+		go = z0 * s3 + (row0 + rg) * n1 + i1;
+		face_rows = 2 * A.nd + 2 * A.RG;
+		lo2 = row0 > 0;
+		hi2 = row0 + nr < A.n2;
+		lo3 = z0 > 0;
+		hi3 = z0 + nd < A.n3;
+	}
+	// A block's faces of a field in global memory: rows i2 low [nd], i2 high
+	// [nd], i3 low [RG], i3 high [RG].
+	__device__ void publish(const ResArgs &A, double *faces, int d, double v) const {
+		if (rg == 0 && lo2) stl2(faces + d * A.n1 + i1, v);
+		if (rg == nr - 1 && hi2) stl2(faces + (A.nd + d) * A.n1 + i1, v);
+		if (d == 0 && lo3) stl2(faces + (2 * A.nd + rg) * A.n1 + i1, v);
+		if (d == nd - 1 && hi3) stl2(faces + (2 * A.nd + A.RG + rg) * A.n1 + i1, v);
+	}
+	// Ghost points of the box, HB rows of a thread at a time: load(k, from) of
+	// the neighbour's face point, then use(k, shared offset).
+	template <int HB, class Load, class Use>
+	__device__ __forceinline__ void ghosts(const ResArgs &A, Load load, Use use) const {
+		if (rg >= A.RG) return;
+		const int n = 2 * nd + 2 * nr;
+		for (int h0 = rg; h0 < n; h0 += HB * A.RG) {
+			int off[HB];
+#pragma unroll
+			for (int k = 0; k < HB; k++) {
+				const int h = h0 + k * A.RG;
+				off[k] = -1;
+				if (h >= n) continue;
+				int j2, j3, fr;  // box row and plane (-1, nr / nd outside), face row of the neighbour
+				bool there;
+				if (h < 2 * nd) {
+					const bool hi = h >= nd;
+					j3 = hi ? h - nd : h;
+					j2 = hi ? nr : -1;
+					there = hi ? hi2 : lo2;
+					fr = hi ? face_rows + j3 : A.nd + j3 - face_rows;
+				} else {
+					const bool hi = h >= 2 * nd + nr;
+					j2 = hi ? h - 2 * nd - nr : h - 2 * nd;
+					j3 = hi ? nd : -1;
+					there = hi ? hi3 : lo3;
+					fr = 2 * A.nd + j2 + (hi ? A.s2 * face_rows : A.RG - A.s2 * face_rows);
+				}
+				if (!there) continue;
+				off[k] = (j3 + 1) * pp + (j2 + 1) * pitch + 1 + i1;
+				load(k, fr * A.n1 + i1);
+			}
+#pragma unroll
+			for (int k = 0; k < HB; k++)
+				if (off[k] >= 0) use(k, off[k]);
+		}
+	}
+	// f(d, centre, A (scale .* field)) of the thread's points; SCALED as the
+	// reference stores the stencil input (each value read times scale).
+	template <int D, bool UNIT, bool SCALED, class F>
+	__device__ __forceinline__ void march(const ResArgs &A, const double *field, double scale, F f) const {
+		if (!own) return;
+		auto in = [&](double v) { return SCALED ? mul(v, scale) : v; };
+		const double *q = field + opaque(so);
+		double prev = in(q[-pp]), raw = q[0], cur = in(raw);
+#pragma unroll
+		for (int d = 0; d < D; d++) {
+			if (d >= nd) break;
+			const double rnext = q[pp], next = in(rnext);
+			f(d, raw, st7r<UNIT>(A.a, A.b, A.c, cur, in(q[-1]), in(q[-pitch]), prev, in(q[1]), in(q[pitch]), next));
+			prev = cur;
+			raw = rnext;
+			cur = next;
+			q += pp;
+		}
+	}
+	// f(d, grid index, b - A x) of the thread's points, x in global memory.
+	template <int D, bool UNIT, class F>
+	__device__ __forceinline__ void residual(const ResArgs &A, const double *x, const double *b, F f) const {
+		if (!own) return;
+		const int n1 = A.n1, i2 = row0 + rg;
+		int i = opaque(go);
+		double prev = z0 > 0 ? ldl2(x + i - s3) : 0.0, cur = ldl2(x + i);
+#pragma unroll
+		for (int d = 0; d < D; d++) {
+			if (d >= nd) break;
+			const double next = z0 + d + 1 < A.n3 ? ldl2(x + i + s3) : 0.0;
+			const double xm1 = i1 > 0 ? ldl2(x + i - 1) : 0.0, xp1 = i1 < n1 - 1 ? ldl2(x + i + 1) : 0.0;
+			const double xm2 = i2 > 0 ? ldl2(x + i - n1) : 0.0, xp2 = i2 < A.n2 - 1 ? ldl2(x + i + n1) : 0.0;
+			const double bi = b[i];
+			f(d, cur, bi, add(bi, -st7r<UNIT>(A.a, A.b, A.c, cur, xm1, xm2, prev, xp1, xp2, next)));
+			prev = cur;
+			cur = next;
+			i += s3;
+		}
+	}
+};
+
+__device__ __forceinline__ void group_init(ResGroup *g, const ResArgs &A) {
+	g->G = A.G;
+	g->m = blockIdx.x % A.G;
+	g->words = A.words + (size_t)(blockIdx.x / A.G) * res_words(A.G);
+	g->err = A.err;
+	g->base = A.stamp;
+	g->fail = 0;
+}
+
+// Uniform state of a pipelined CG or BiCGStab solve, in shared memory: warp 0
+// writes it at the end of a group sum.
+struct KrylovState {
+	double bb, rr, err, alpha, beta;
+	double gamma, gamma_old, delta;              // pipelined CG
+	double rho, rho_prev, omega, bo, s_norm2;    // BiCGStab
+	int done, reason, ex, s_exit;
+};
+
+__device__ __forceinline__ void stop(KrylovState &st, int reason, int ex) {
+	st.done = 1;
+	st.reason = reason;
+	st.ex = ex;
+}
+
+// <b,b>, <r,r>: the initial error and test (Cg.hpp:112-134 and its twins).
+__device__ __forceinline__ void initial_state(KrylovState &st, const ResArgs &A, double bb, double rr, bool hist) {
+	st.bb = bb == 0.0 ? 1.0 : bb;
+	st.rr = rr;
+	st.err = sqrt(__ddiv_rn(rr, st.bb));
+	st.done = st.s_exit = 0;
+	st.reason = STOP_NONE;
+	st.ex = 0;
+	st.s_norm2 = st.rho_prev = 0.0;
+	st.omega = 1.0;  // BiCgStab.hpp:147-150
+	st.alpha = st.beta = 0.0;
+	if (hist) A.hist[0] = st.err;
+	if (st.err < A.tol) stop(st, STOP_EARLY, 0);
+	else if (A.maxiter < 1) stop(st, STOP_MAXITER, 1);
+}
+
+__device__ __forceinline__ void write_state(const KrylovState &st, const ResArgs &A, int k) {
+	A.o_err[k] = st.err;
+	A.o_bb[k] = st.bb;
+	A.o_rr[k] = st.rr;
+	A.o_exit[k] = st.ex;
+	A.o_reason[k] = st.reason;
+	A.o_done[k] = 1;
+	if (A.o_snorm) {
+		A.o_snorm[k] = st.s_norm2;
+		A.o_omega[k] = st.omega;
+		A.o_rho[k] = st.rho;
+	}
+}
+
+// ---------------------------------------------------------------------------
+// Pipelined CG (PipelinedCg.hpp:136-230), FP64.  Shared memory holds m = w .*
+// iM with its ghosts and the thread's own points of q, s, p, z and x; r, u and
+// w are in registers.  An iteration is one stencil pass with the eight updates
+// and one group reduction, which also publishes the boundary rows of m.
+// ---------------------------------------------------------------------------
+template <int D, bool UNIT>
+__global__ void __launch_bounds__(512, 1) k_res_pcg(const __grid_constant__ ResArgs A) {
+	extern __shared__ __align__(16) unsigned char smem[];
+	__shared__ ResGroup gsh;
+	__shared__ KrylovState st;
+	ResGroup *const g = &gsh;
+	const ResBox B(A);
+	const int t = threadIdx.x, T = blockDim.x;
+	const int elems = B.pp * (A.nd + 2) + 1;
+	double *const sm = reinterpret_cast<double *>(smem);
+	double *const fq = sm + elems + t, *const fs = fq + A.nd * T, *const fp = fs + A.nd * T, *const fz = fp + A.nd * T,
+	             *const fx = fz + A.nd * T;  // own point of plane d at [d * T]
+	// The faces of two rounds: a block publishes new rows while a neighbour may
+	// still read the old ones.
+	double *const faces = static_cast<double *>(A.edge) + (size_t)blockIdx.x * B.face_rows * A.n1;
+	const size_t other = (size_t)gridDim.x * B.face_rows * A.n1;
+	if (t == 0) group_init(g, A);
+	unsigned round = 0;
+	const double im = A.iM;
+	for (int unit = blockIdx.x / A.G; unit < A.lanes; unit += A.groups) {
+		double *const x = A.x + (size_t)unit * A.npts;
+		const bool hist = A.hist && unit == 0 && blockIdx.x % A.G == 0;
+		const double *in = faces;     // read
+		double *out = faces + other;  // published next
+		for (int e = t; e < elems; e += T) sm[e] = 0.0;
+		__syncthreads();
+		double r[D], u[D], w[D];
+		{
+			double v[2] = {0.0, 0.0};
+			B.residual<D, UNIT>(A, x, A.rhs + (size_t)unit * A.npts, [&](int d, double xi, double bi, double ri) {
+				r[d] = ri;
+				u[d] = mul(ri, im);  // :138
+				fx[d * T] = xi;
+				fq[d * T] = fs[d * T] = fp[d * T] = fz[d * T] = 0.0;  // :146-149
+				sm[B.so + d * B.pp] = u[d];
+				B.publish(A, faces, d, u[d]);
+				v[0] = fma(bi, bi, v[0]);
+				v[1] = fma(ri, ri, v[1]);
+			});
+			if (!group_sum<2, true>(g, round, v, Nothing(), [&](int lane, const double (&tot)[2]) {
+				    if (lane == 0) initial_state(st, A, tot[0], tot[1], hist);
+			    }))
+				return;
+		}
+		constexpr int HB = 6;
+		double hv[HB];
+		auto load = [&](int k, int from) { hv[k] = ldl2(in + from); };
+		auto put = [&](int k, int off) { sm[off] = hv[k]; };
+		// fin of a sum of <r,u>, <w,u>, <r,r>: the scalars of the next iteration (:175-181).
+		auto next_scalars = [&](const double (&tot)[3], bool first) {
+			st.gamma_old = st.gamma;
+			st.gamma = tot[0];
+			st.delta = tot[1];
+			st.rr = tot[2];
+			if (first) {
+				st.beta = 0.0;
+				st.alpha = __ddiv_rn(tot[0], tot[1]);
+			} else {
+				st.beta = __ddiv_rn(tot[0], st.gamma_old);
+				st.alpha = __ddiv_rn(1.0, __dsub_rn(__ddiv_rn(tot[1], tot[0]), __ddiv_rn(st.beta, st.alpha)));
+			}
+		};
+		if (!st.done) {
+			B.ghosts<HB>(A, load, put);
+			__syncthreads();
+			double v[3] = {0.0, 0.0, 0.0};
+			B.march<D, UNIT, false>(A, sm, 1.0, [&](int d, double, double wi) {  // w = A u (:141-143)
+				w[d] = wi;
+				v[0] = fma(r[d], u[d], v[0]);
+				v[1] = fma(wi, u[d], v[1]);
+				v[2] = fma(r[d], r[d], v[2]);
+				B.publish(A, out, d, mul(wi, im));
+			});
+			auto new_m = [&]() {  // m = w .* iM (:158): every thread has left the stencil pass
+				if (B.own)
+#pragma unroll
+					for (int d = 0; d < D; d++)
+						if (d < B.nd) sm[B.so + d * B.pp] = mul(w[d], im);
+			};
+			if (!group_sum<3, true>(g, round, v, new_m, [&](int lane, const double (&tot)[3]) {
+				    if (lane == 0) next_scalars(tot, true);
+			    }))
+				return;
+			for (int it = 1; !st.done; it++) {
+				in = faces + (it & 1) * other;
+				out = faces + (~it & 1) * other;
+				B.ghosts<HB>(A, load, put);
+				__syncthreads();
+				const double alpha = st.alpha, beta = st.beta;
+				v[0] = v[1] = v[2] = 0.0;
+				B.march<D, UNIT, false>(A, sm, 1.0, [&](int d, double mi, double ni) {  // n = A m (:161-184)
+					const double qi = add(mi, mul(beta, fq[d * T]));      // :200
+					const double si = add(w[d], mul(beta, fs[d * T]));    // :203
+					const double pi = add(u[d], mul(beta, fp[d * T]));    // :206
+					const double zi = add(ni, mul(beta, fz[d * T]));      // :209
+					fq[d * T] = qi;
+					fs[d * T] = si;
+					fp[d * T] = pi;
+					fz[d * T] = zi;
+					r[d] = add(r[d], mul(-alpha, si));                    // :212
+					fx[d * T] = add(fx[d * T], mul(alpha, pi));           // :215
+					u[d] = add(u[d], mul(-alpha, qi));                    // :218
+					w[d] = add(w[d], mul(-alpha, zi));                    // :221
+					B.publish(A, out, d, mul(w[d], im));
+					v[0] = fma(r[d], u[d], v[0]);
+					v[1] = fma(w[d], u[d], v[1]);
+					v[2] = fma(r[d], r[d], v[2]);
+				});
+				if (!group_sum<3, true>(g, round, v, new_m, [&](int lane, const double (&tot)[3]) {
+					    if (lane != 0) return;
+					    // The stop test uses <r,r> from the top of this iteration (:173, :227).
+					    const double rr = st.rr;
+					    st.err = sqrt(__ddiv_rn(rr, st.bb));
+					    if (hist) A.hist[it] = st.err;
+					    if (st.err <= A.tol_in) stop(st, STOP_CONVERGED, it);
+					    else if (it >= A.maxiter) stop(st, STOP_MAXITER, A.maxiter + 1);
+					    if (st.done) st.rr = rr;
+					    else next_scalars(tot, false);
+				    }))
+					return;
+			}
+			if (B.own)
+				for (int d = 0; d < B.nd; d++) stl2(x + B.go + d * B.s3, fx[d * T]);
+		}
+		if (blockIdx.x % A.G == 0 && t == 0) write_state(st, A, unit);
+		__syncthreads();  // shared memory is reused by the next right-hand side
+	}
+}
+
+// ---------------------------------------------------------------------------
+// BiCGStab (BiCgStab.hpp:157-232), FP64.  Shared memory holds p and s with
+// their ghosts and the thread's own points of x and r_hat; r, v and t are in
+// registers.  Three group reductions an iteration; the first publishes the
+// boundary rows of v, the third those of r, and every block forms its ghosts
+// of p and s from them (times iM at each read, as the reference rounds p_hat
+// and s_hat).
+// ---------------------------------------------------------------------------
+template <int D, bool UNIT>
+__global__ void __launch_bounds__(512, 1) k_res_bicg(const __grid_constant__ ResArgs A) {
+	extern __shared__ __align__(16) unsigned char smem[];
+	__shared__ ResGroup gsh;
+	__shared__ KrylovState st;
+	ResGroup *const g = &gsh;
+	const ResBox B(A);
+	const int t = threadIdx.x, T = blockDim.x;
+	const int elems = B.pp * (A.nd + 2) + 1;
+	double *const sp = reinterpret_cast<double *>(smem), *const ss = sp + elems;
+	double *const fx = ss + elems + t, *const fh = fx + A.nd * T;  // own x, r_hat of plane d at [d * T]
+	double *const rfaces = static_cast<double *>(A.edge) + (size_t)blockIdx.x * B.face_rows * A.n1;
+	// v's faces of two iterations: a block publishes new rows while a neighbour
+	// may still form its p from the old ones.
+	const size_t other = (size_t)gridDim.x * B.face_rows * A.n1;
+	const double *vin = nullptr;
+	if (t == 0) group_init(g, A);
+	unsigned round = 0;
+	const double im = A.iM;
+	constexpr int HB = 4;
+	double hr[HB], hw[HB];
+	auto load_r = [&](int k, int from) { hr[k] = ldl2(rfaces + from); };
+	auto load_rv = [&](int k, int from) {
+		hr[k] = ldl2(rfaces + from);
+		hw[k] = ldl2(vin + from);
+	};
+	for (int unit = blockIdx.x / A.G; unit < A.lanes; unit += A.groups) {
+		double *const x = A.x + (size_t)unit * A.npts;
+		const bool hist = A.hist && unit == 0 && blockIdx.x % A.G == 0;
+		for (int e = t; e < 2 * elems; e += T) sp[e] = 0.0;
+		__syncthreads();
+		double r[D], vv[D], tt[D];
+		{
+			double v[2] = {0.0, 0.0};
+			B.residual<D, UNIT>(A, x, A.rhs + (size_t)unit * A.npts, [&](int d, double xi, double bi, double ri) {
+				r[d] = ri;
+				fx[d * T] = xi;
+				fh[d * T] = ri;  // r_hat = r (:153)
+				B.publish(A, rfaces, d, ri);
+				v[0] = fma(bi, bi, v[0]);
+				v[1] = fma(ri, ri, v[1]);
+			});
+			if (!group_sum<2, true>(g, round, v, Nothing(), [&](int lane, const double (&tot)[2]) {
+				    if (lane != 0) return;
+				    initial_state(st, A, tot[0], tot[1], hist);
+				    st.rho = tot[1];  // <r, r_hat> with r_hat == r (:159-160)
+				    if (!st.done && st.rho == 0.0) stop(st, STOP_RHO, 1);
+			    }))
+				return;
+		}
+		for (int it = 1; !st.done; it++) {
+			// ---- 1: p = r + beta p - beta omega v (p = r first), v = A p_hat, <v, r_hat>.
+			double *const vnew = rfaces + (1 + (it & 1)) * other;
+			vin = rfaces + (1 + (~it & 1)) * other;
+			{
+				const bool first = it == 1;
+				const double beta = st.beta, bo = st.bo;
+				auto new_p = [&](double ri, double pi, double vi) {
+					return first ? ri : add(add(ri, mul(beta, pi)), mul(bo, vi));  // :168, :171
+				};
+				if (first) B.ghosts<HB>(A, load_r, [&](int k, int off) { sp[off] = hr[k]; });
+				else B.ghosts<HB>(A, load_rv, [&](int k, int off) { sp[off] = new_p(hr[k], sp[off], hw[k]); });
+				if (B.own)
+#pragma unroll
+					for (int d = 0; d < D; d++)
+						if (d < B.nd) {
+							double *const p = sp + B.so + d * B.pp;
+							*p = new_p(r[d], *p, first ? 0.0 : vv[d]);
+						}
+				__syncthreads();
+				double v[1] = {0.0};
+				B.march<D, UNIT, true>(A, sp, im, [&](int d, double, double vi) {  // :178-180
+					vv[d] = vi;
+					v[0] = fma(vi, fh[d * T], v[0]);
+					B.publish(A, vnew, d, vi);
+				});
+				if (!group_sum<1, true>(g, round, v, Nothing(), [&](int lane, const double (&tot)[1]) {
+					    if (lane == 0) st.alpha = __ddiv_rn(st.rho, tot[0]);  // :186
+				    }))
+					return;
+			}
+			// ---- 2: s = r - alpha v, t = A s_hat; <s,s>, <t,s>, <t,t>.
+			const double alpha = st.alpha;
+			vin = vnew;
+			{
+				B.ghosts<HB>(A, load_rv, [&](int k, int off) { ss[off] = add(hr[k], mul(-alpha, hw[k])); });  // :189
+				if (B.own)
+#pragma unroll
+					for (int d = 0; d < D; d++)
+						if (d < B.nd) ss[B.so + d * B.pp] = add(r[d], mul(-alpha, vv[d]));
+				__syncthreads();
+				double v[3] = {0.0, 0.0, 0.0};
+				B.march<D, UNIT, true>(A, ss, im, [&](int d, double si, double ti) {  // :204-206
+					tt[d] = ti;
+					v[0] = fma(si, si, v[0]);
+					v[1] = fma(ti, si, v[1]);
+					v[2] = fma(ti, ti, v[2]);
+				});
+				if (!group_sum<3>(g, round, v, Nothing(), [&](int lane, const double (&tot)[3]) {
+					    if (lane != 0) return;
+					    st.s_norm2 = tot[0];  // :192-193
+					    st.s_exit = tot[0] < __dmul_rn(A.tol_in, A.tol_in);  // :194
+					    if (!st.s_exit) st.omega = __ddiv_rn(tot[1], tot[2]);  // :212
+				    }))
+					return;
+			}
+			// ---- 3: x += alpha p_hat (+ omega s_hat), r = s - omega t; <r,r>, <r, r_hat>.
+			const double omega = st.omega;
+			const bool s_exit = st.s_exit != 0;
+			double v[2] = {0.0, 0.0};
+			if (B.own)
+#pragma unroll
+				for (int d = 0; d < D; d++) {
+					if (d >= B.nd) break;
+					const double ph = mul(sp[B.so + d * B.pp], im), si = ss[B.so + d * B.pp];
+					const double x1 = add(fx[d * T], mul(alpha, ph));
+					if (s_exit) {
+						fx[d * T] = x1;  // :196
+						continue;
+					}
+					fx[d * T] = add(x1, mul(omega, mul(si, im)));  // :216
+					r[d] = add(si, mul(-omega, tt[d]));            // :219
+					B.publish(A, rfaces, d, r[d]);
+					v[0] = fma(r[d], r[d], v[0]);
+					v[1] = fma(r[d], fh[d * T], v[1]);
+				}
+			if (!group_sum<2, true>(g, round, v, Nothing(), [&](int lane, const double (&tot)[2]) {
+				    if (lane != 0) return;
+				    if (s_exit) {
+					    stop(st, STOP_SNORM, it);
+					    return;
+				    }
+				    st.rr = tot[0];
+				    st.err = sqrt(__ddiv_rn(tot[0], st.bb));  // :226
+				    if (hist) A.hist[it] = st.err;
+				    if (st.err <= A.tol_in) {                   // :228
+					    stop(st, STOP_CONVERGED, it);
+				    } else if (omega == 0.0) {                  // :229
+					    stop(st, STOP_OMEGA, it);
+				    } else {
+					    st.rho_prev = st.rho;                    // :231
+					    if (it >= A.maxiter) {
+						    stop(st, STOP_MAXITER, A.maxiter + 1);
+					    } else {
+						    st.rho = tot[1];                     // next iteration :159-160
+						    if (tot[1] == 0.0) stop(st, STOP_RHO, it + 1);  // :162
+						    st.beta = __dmul_rn(__ddiv_rn(st.rho, st.rho_prev), __ddiv_rn(st.alpha, st.omega));  // :166
+						    st.bo = __dmul_rn(-st.beta, st.omega);
+					    }
+				    }
+			    }))
+				return;
+		}
+		if (st.reason != STOP_EARLY && B.own)
+			for (int d = 0; d < B.nd; d++) stl2(x + B.go + d * B.s3, fx[d * T]);
+		if (blockIdx.x % A.G == 0 && t == 0) write_state(st, A, unit);
+		__syncthreads();  // shared memory is reused by the next right-hand side
+	}
+}
+
 }  // namespace
 
 // ---------------------------------------------------------------------------
@@ -693,10 +1167,15 @@ namespace {
 typedef void (*ResKernel)(const ResArgs);
 
 // Box shapes: C rows x at most D planes per thread, at most T threads, so many
-// blocks per SM.
-constexpr int kShapes = 6;
-constexpr int kShapeC[kShapes] = {1, 1, 2, 2, 3, 2}, kShapeD[kShapes] = {2, 8, 8, 16, 16, 16},
-              kShapeT[kShapes] = {512, 512, 512, 512, 384, 256}, kShapeB[kShapes] = {1, 1, 1, 1, 1, 2};
+// blocks per SM.  The last ones, one row per thread, are those of pipelined CG
+// and BiCGStab.
+constexpr int kShapes = 9, kCgShapes = 6;
+constexpr int kShapeC[kShapes] = {1, 1, 2, 2, 3, 2, 1, 1, 1}, kShapeD[kShapes] = {2, 8, 8, 16, 16, 16, 2, 4, 8},
+              kShapeT[kShapes] = {512, 512, 512, 512, 384, 256, 512, 512, 512},
+              kShapeB[kShapes] = {1, 1, 1, 1, 1, 2, 1, 1, 1};
+// Fields of a solver in shared memory with ghosts, and own points only; fields
+// whose faces it publishes.
+constexpr int kGhosted[4] = {0, 2, 1, 1}, kOwn[4] = {0, 2, 0, 5}, kFaces[4] = {0, 3, 1, 2};  // by solver id
 
 template <class V, bool UNIT>
 ResKernel cg_kernel(int shape) {
@@ -710,7 +1189,17 @@ ResKernel cg_kernel(int shape) {
 	}
 }
 
-ResKernel kernel_for(bool fp32, bool unit, int shape) {
+template <bool UNIT>
+ResKernel krylov_kernel(int ks, int shape) {
+	switch (shape) {
+	case 6: return ks == SEDI_BICGSTAB ? (ResKernel)k_res_bicg<2, UNIT> : (ResKernel)k_res_pcg<2, UNIT>;
+	case 7: return ks == SEDI_BICGSTAB ? (ResKernel)k_res_bicg<4, UNIT> : (ResKernel)k_res_pcg<4, UNIT>;
+	default: return ks == SEDI_BICGSTAB ? (ResKernel)k_res_bicg<8, UNIT> : (ResKernel)k_res_pcg<8, UNIT>;
+	}
+}
+
+ResKernel kernel_for(int ks, bool fp32, bool unit, int shape) {
+	if (ks != SEDI_CG) return unit ? krylov_kernel<true>(ks, shape) : krylov_kernel<false>(ks, shape);
 	if (fp32) return cg_kernel<float2, false>(shape);  // FP32 folds b, c into its multiply-adds
 	return unit ? cg_kernel<double, true>(shape) : cg_kernel<double, false>(shape);
 }
@@ -726,20 +1215,25 @@ struct Plan {
 // a point adds 1.3 where A p stays in registers (2048 points a block 13600, 8192
 // 20100), 1.65 with two stencil passes (16384: 38000), 1.8 at three rows a
 // thread (12672: 32500), and 3.2 with two blocks on an SM (2 x 8192: 37400).
-Plan plan_for(const Geo &g, int units, int sms, size_t smem_max, double *cycles) {
-	constexpr double kPoint[kShapes] = {1.3, 1.3, 1.3, 1.65, 1.8, 3.2};
+// Pipelined CG: 256 points a block 7700, 2048 10400, 4096 14000; BiCGStab: 512
+// points 19000, 2048 24000, 4096 29000.
+Plan plan_for(int ks, const Geo &g, int units, int sms, size_t smem_max, double *cycles) {
+	constexpr double kPoint[kCgShapes] = {1.3, 1.3, 1.3, 1.65, 1.8, 3.2};
+	constexpr double kSync[4] = {0.0, 16000.0, 9000.0, 6000.0}, kPointOf[4] = {0.0, 2.9, 0.0, 1.6};  // by solver id
 	Plan best;
-	for (int sh = 0; sh < kShapes; sh++) {
+	for (int sh = ks == SEDI_CG ? 0 : kCgShapes; sh < (ks == SEDI_CG ? kCgShapes : kShapes); sh++) {
 		const int C = kShapeC[sh], slots = sms * kShapeB[sh];  // blocks at once
 		for (int RG = kShapeT[sh] / g.n1; RG >= 1; RG--) {
 			if (RG > 1 && (RG - 1) * C >= g.n2) continue;  // a row group with nothing to do
 			const int T = (RG * g.n1 + 31) / 32 * 32, B2 = RG * C, s2 = (g.n2 + B2 - 1) / B2;
 			for (int nd = 1; nd <= kShapeD[sh] && nd <= g.n3; nd++) {
 				const long long G = (long long)s2 * ((g.n3 + nd - 1) / nd);
-				const size_t smem = ((size_t)(g.n1 + 1) * (B2 + 2) * (nd + 2) + 1) * 8;
+				const size_t smem = (((size_t)(g.n1 + 1) * (B2 + 2) * (nd + 2) + 1) * kGhosted[ks] + (size_t)kOwn[ks] * nd * T) * 8;
 				if (G > slots || smem * kShapeB[sh] > smem_max) continue;
 				const int groups = units < slots / (int)G ? units : slots / (int)G;
-				const double cost = ((G > 1 ? 9000.0 + 15.0 * G : 3000.0) + kPoint[sh] * T * C * nd) *
+				const double point = ks == SEDI_CG ? kPoint[sh < kCgShapes ? sh : 0] : kPointOf[ks];
+				const double deep = ks != SEDI_CG && nd > 4 ? 1500.0 : 0.0;  // the 8-plane kernels' start-up
+				const double cost = ((G > 1 ? kSync[ks] + 15.0 * G : kSync[ks] / 3.0) + deep + point * T * C * nd) *
 				                    ((units + groups - 1) / groups);
 				if (best.shape >= 0 && cost >= *cycles) continue;
 				*cycles = cost;
@@ -758,25 +1252,29 @@ Plan plan_for(const Geo &g, int units, int sms, size_t smem_max, double *cycles)
 }
 
 // Estimated time of an iteration of the streaming sweeps on a batch, in cycles
-// of the same clock: launches and latency, then HBM (CG: 7.5 words per point
-// and lane), more where the tiles overhang the grid.  Measured (us): FP64
+// of the same clock: launches and latency, then HBM (words per point and lane;
+// BiCGStab's 15 at five sixths of CG's rate), more where the tiles overhang
+// the grid.  Measured (us): pipelined CG 32^3 x 64 60, 64^3 x 64 374; BiCGStab
+// 82, 457; CG FP64
 // 32^3 x 16 27, 64^3 x 64 188, 96^3 x 64 578, 128^3 x 64 1418; FP32 64^3 x 64
 // 122, 96^3 x 64 320, 128^3 x 64 798.
-double stream_cycles(const Geo &g, int lanes, bool fp32) {
+double stream_cycles(int ks, const Geo &g, int lanes, bool fp32) {
 	const double over = (double)((g.n1 + 31) / 32 * 32) * ((g.n2 + 31) / 32 * 32) / ((double)g.n1 * g.n2);
-	return 1950.0 * (26.0 + 7.5 * (fp32 ? 4.0 : 8.0) * (double)g.n * lanes * std::sqrt(over) / 5.9e6);
+	constexpr double kLaunch[4] = {0.0, 42.0, 26.0, 18.0}, kWords[4] = {0.0, 18.0, 7.5, 16.0};  // by solver id
+	return 1950.0 * (kLaunch[ks] + kWords[ks] * (fp32 ? 4.0 : 8.0) * (double)g.n * lanes * std::sqrt(over) / 5.9e6);
 }
 
 size_t word_bytes(const Plan &p) { return sizeof(Word2) * res_words(p.G) * p.groups; }
 
-size_t edge_bytes(const Plan &p, const Geo &g) {
-	return 8 * (size_t)p.groups * p.G * (2 * p.nd + 2 * p.RG * kShapeC[p.shape]) * g.n1;
+size_t edge_bytes(int ks, const Plan &p, const Geo &g) {
+	return 8 * (size_t)kFaces[ks] * (size_t)p.groups * p.G * (2 * p.nd + 2 * p.RG * kShapeC[p.shape]) * g.n1;
 }
 
 }  // namespace
 
 struct Resident {
 	Plan plan;
+	int ks = 0;
 	bool fp32 = false, unit = false;
 	Word2 *words = nullptr;
 	void *edge = nullptr;
@@ -808,7 +1306,7 @@ static void running_remove(Resident *R) {
 // and march kernels serve those).
 int resident_alloc(Ctx *c, int ks, bool fp32, int lanes, Resident **out) {
 	*out = nullptr;
-	if (ks != SEDI_CG) return 0;
+	if (ks != SEDI_CG && fp32) return 0;
 	if (c->g.n1 > 512 || c->g.n > (1 << 22)) return 0;  // no box shape takes them
 	int sms = 0, coop = 0, smem_max = 0;
 	const bool unit = c->k.b == 1.0 && c->k.c == 1.0;
@@ -822,15 +1320,15 @@ int resident_alloc(Ctx *c, int ks, bool fp32, int lanes, Resident **out) {
 	const size_t shared = (size_t)smem_max - 2 * (sizeof(ResGroup) + sizeof(CgState<2>) + 1024);
 	if (sms > kResMaxBlocks / 2) sms = kResMaxBlocks / 2;
 	double cycles = 0.0;
-	const Plan p = plan_for(c->g, fp32 ? (lanes + 1) / 2 : lanes, sms, shared, &cycles);
+	const Plan p = plan_for(ks, c->g, fp32 ? (lanes + 1) / 2 : lanes, sms, shared, &cycles);
 	if (p.shape < 0) return 0;
 	// A pair of FP32 lanes takes 1.6-1.9 times an FP64 lane (conversions for its
 	// FP64 sums).  One right-hand side has no streaming form at these sizes
 	// (its march kernels take 12 us an iteration at 32^3, 47 at 128^3; this 5.6
 	// and 20), a batch does.
 	if (fp32) cycles *= 1.8;
-	if (lanes > 1 && cycles > stream_cycles(c->g, lanes, fp32)) return 0;
-	const ResKernel k = kernel_for(fp32, unit, p.shape);
+	if (lanes > 1 && cycles > stream_cycles(ks, c->g, lanes, fp32)) return 0;
+	const ResKernel k = kernel_for(ks, fp32, unit, p.shape);
 	int per_sm = 0;
 	// (The attribute is the kernel's, whoever launches it: its largest use.)
 	if (cudaFuncSetAttribute((const void *)k, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -842,11 +1340,12 @@ int resident_alloc(Ctx *c, int ks, bool fp32, int lanes, Resident **out) {
 	Resident *R = new (std::nothrow) Resident();
 	if (!R) return SEDI_ERR_NOMEM;
 	R->plan = p;
+	R->ks = ks;
 	R->fp32 = fp32;
 	R->unit = unit;
 	R->device = c->device;
 	R->sms = sms;
-	if (cudaMalloc(&R->words, word_bytes(p)) != cudaSuccess || cudaMalloc(&R->edge, edge_bytes(p, c->g)) != cudaSuccess ||
+	if (cudaMalloc(&R->words, word_bytes(p)) != cudaSuccess || cudaMalloc(&R->edge, edge_bytes(ks, p, c->g)) != cudaSuccess ||
 	    cudaEventCreateWithFlags(&R->done, cudaEventDisableTiming) != cudaSuccess) {
 		cudaGetLastError();
 		resident_free(R);
@@ -855,7 +1354,7 @@ int resident_alloc(Ctx *c, int ks, bool fp32, int lanes, Resident **out) {
 	}
 	// No word may carry a stamp of a launch to come.
 	cudaMemsetAsync(R->words, 0, word_bytes(p), c->stream);
-	cudaMemsetAsync(R->edge, 0, edge_bytes(p, c->g), c->stream);
+	cudaMemsetAsync(R->edge, 0, edge_bytes(ks, p, c->g), c->stream);
 	*out = R;
 	return cudaStreamSynchronize(c->stream) == cudaSuccess ? 0 : set_cuda_error(c, cudaGetLastError(), "resident_alloc");
 }
@@ -908,6 +1407,9 @@ int resident_launch(Ctx *c, Resident *R, const ResIO &io) {
 	a.o_exit = io.o_exit;
 	a.o_reason = io.o_reason;
 	a.o_done = io.o_done;
+	a.o_snorm = io.o_snorm;
+	a.o_omega = io.o_omega;
+	a.o_rho = io.o_rho;
 	a.hist = io.hist;
 	a.err = io.err;
 	void *args[] = {&a};
@@ -933,7 +1435,7 @@ int resident_launch(Ctx *c, Resident *R, const ResIO &io) {
 		if (w != cudaSuccess) return set_cuda_error(c, w, "resident solver launch");
 		held -= o->held;
 	}
-	cudaError_t e = cudaLaunchCooperativeKernel((const void *)kernel_for(R->fp32, R->unit, p.shape), dim3((unsigned)blocks),
+	cudaError_t e = cudaLaunchCooperativeKernel((const void *)kernel_for(R->ks, R->fp32, R->unit, p.shape), dim3((unsigned)blocks),
 	                                            dim3((unsigned)p.T), args, p.smem, c->stream);
 	if (e == cudaSuccess && need > 0) {
 		e = cudaEventRecord(R->done, c->stream);

@@ -153,6 +153,7 @@ struct ResIO {
 	int maxiter, period;
 	double *o_err, *o_bb, *o_rr;  // device, per right-hand side
 	int *o_exit, *o_reason, *o_done;
+	double *o_snorm, *o_omega, *o_rho;  // BiCGStab
 	double *hist;
 	int *err;
 };

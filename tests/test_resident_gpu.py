@@ -20,21 +20,36 @@ pytestmark = pytest.mark.gpu
 # block row (512), one point wide, every box shape's size range, and the first
 # grid that is too wide (513).
 @pytest.mark.parametrize("dims", [(33, 17, 9), (97, 65, 51), (128, 33, 70), (512, 6, 5), (513, 4, 3), (1, 40, 37),
-                                  (31, 1, 64), (64, 64, 64), (300, 40, 30), (100, 110, 120)])
+                                  (31, 1, 64), (64, 64, 64), (300, 40, 30), (100, 110, 120), (80, 85, 88)])
 @pytest.mark.parametrize("coeffs", [(6.0, 1.0, 1.0), (6.5, 1.2, 0.9)])
-def test_single_vector_matches_oracle(dims, coeffs):
+@pytest.mark.parametrize("solver,K", [("cg", 21), ("pcg", 21), ("bicgstab", 12)])
+def test_single_vector_matches_oracle(dims, coeffs, solver, K):
     n = int(np.prod(dims))
     b = O.fill_probe(7, n)
     x0 = np.cos(np.arange(n))
-    K = 21
-    rc0, fe0, fi0, xo, h0 = O.solve(2, dims, b, x0=x0, maxiter=K, tol=0.0, coeffs=coeffs)
+    rc0, fe0, fi0, xo, h0 = O.solve(S.SOLVER_IDS[solver], dims, b, x0=x0, maxiter=K, tol=0.0, coeffs=coeffs)
     x = x0.copy()
-    with S.Context("cg", dims, S.Stencil(*coeffs)) as c:
+    with S.Context(solver, dims, S.Stencil(*coeffs)) as c:
         rc, fe, fi = c.solve(x, b, None, K, 0.0)
         hist = c.history()
     assert (rc, fi) == (rc0, fi0)
     assert O.relmax(x, xo) <= 1e-10
     assert len(hist) == len(h0[:K + 1]) and O.relmax(hist, h0[:K + 1]) <= 1e-9
+
+
+@pytest.mark.parametrize("solver,K", [("pcg", 25), ("bicgstab", 12)])
+@pytest.mark.parametrize("dims,lanes", [((33, 17, 9), 5), ((40, 36, 30), 40), ((64, 20, 50), 3)])
+def test_fp64_batches_match_single_vector(dims, lanes, solver, K):
+    n = int(np.prod(dims))
+    B = np.stack([O.fill_probe(90 + k, n) for k in range(lanes)])
+    X = np.zeros_like(B)
+    with S.Context(solver, dims, batch=lanes) as c:
+        res, fe, fi = c.solve_batch(X, B, maxiter=K, tol=0.0)
+    with S.Context(solver, dims) as c:
+        for k in (0, lanes // 2, lanes - 1):
+            x = np.zeros(n)
+            out = c.solve(x, B[k], None, K, 0.0)
+            assert (res[k], fi[k]) == (out[0], out[2]) and O.relmax(X[k], x) <= 1e-10
 
 
 @pytest.mark.parametrize("prec", [S.FP64, S.MIXED])
