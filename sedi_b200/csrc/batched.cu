@@ -2383,6 +2383,10 @@ static int resident_chunk(Ctx *c, Batched *B) {
 	io.rhs = B->rhs;
 	io.x = B->mixed ? B->xh : (double *)B->x;
 	io.xlo = B->mixed ? B->x : nullptr;
+	io.scratch[0] = (double *)B->q;
+	io.scratch[1] = (double *)B->sv;
+	io.scratch[2] = (double *)B->p0;
+	io.scratch[3] = (double *)B->z;
 	io.tol = g0.tol;
 	io.tol_in = g0.tol_in;
 	io.maxiter = g0.maxiter;

@@ -657,6 +657,10 @@ static int resident_solve(Ctx *c, const double *b, double *x, int maxiter, doubl
 	io.lanes = 1;
 	io.rhs = b;
 	io.x = x;
+	io.scratch[0] = c->q;
+	io.scratch[1] = c->s;
+	io.scratch[2] = c->p[0];
+	io.scratch[3] = c->z;
 	io.tol = io.tol_in = tol;
 	io.maxiter = maxiter;
 	io.o_err = &c->st->err;

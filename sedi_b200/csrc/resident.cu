@@ -44,6 +44,8 @@ struct ResArgs {
 	void *edge;           // boundary rows: [fields][groups][G][2 nd + 2 RG*C][n1] of V
 	Word2 *words;         // [groups][res_words(G)]: the groups' reductions
 	unsigned long long stamp;  // stamps of this launch lie above it
+	double *scratch[4];   // own-point fields that do not fit shared memory: q, s, p, z (pipelined CG)
+	int nsm;              // own-point fields that do
 	double tol, tol_in;   // stop targets (tol_in = theta * tol for FP32)
 	int maxiter, period;
 	double *o_err, *o_bb, *o_rr;  // per right-hand side
@@ -858,10 +860,12 @@ __device__ __forceinline__ void write_state(const KrylovState &st, const ResArgs
 // Pipelined CG (PipelinedCg.hpp:136-230), FP64.  Shared memory holds m = w .*
 // iM with its ghosts and the thread's own points of q, s, p, z and x; r, u and
 // w are in registers.  An iteration is one stencil pass with the eight updates
-// and one group reduction, which also publishes the boundary rows of m.
+// and one group reduction, which also publishes the boundary rows of m.  Boxes
+// of more than 8 planes keep in shared memory what fits (A.nsm fields) and the
+// other own points in global memory, that is in L2.
 // ---------------------------------------------------------------------------
-template <int D, bool UNIT>
-__global__ void __launch_bounds__(512, 1) k_res_pcg(const __grid_constant__ ResArgs A) {
+template <int D, int TMAX, bool UNIT>
+__global__ void __launch_bounds__(TMAX, 1) k_res_pcg(const __grid_constant__ ResArgs A) {
 	extern __shared__ __align__(16) unsigned char smem[];
 	__shared__ ResGroup gsh;
 	__shared__ KrylovState st;
@@ -870,8 +874,7 @@ __global__ void __launch_bounds__(512, 1) k_res_pcg(const __grid_constant__ ResA
 	const int t = threadIdx.x, T = blockDim.x;
 	const int elems = B.pp * (A.nd + 2) + 1;
 	double *const sm = reinterpret_cast<double *>(smem);
-	double *const fq = sm + elems + t, *const fs = fq + A.nd * T, *const fp = fs + A.nd * T, *const fz = fp + A.nd * T,
-	             *const fx = fz + A.nd * T;  // own point of plane d at [d * T]
+	constexpr bool GLOBAL = D > 8;
 	// The faces of two rounds: a block publishes new rows while a neighbour may
 	// still read the old ones.
 	double *const faces = static_cast<double *>(A.edge) + (size_t)blockIdx.x * B.face_rows * A.n1;
@@ -884,6 +887,19 @@ __global__ void __launch_bounds__(512, 1) k_res_pcg(const __grid_constant__ ResA
 		const bool hist = A.hist && unit == 0 && blockIdx.x % A.G == 0;
 		const double *in = faces;     // read
 		double *out = faces + other;  // published next
+		// Own point of plane d of field k (q, s, p, z, x).
+		double *own[5];
+		int step[5];
+#pragma unroll
+		for (int k = 0; k < 5; k++) {
+			own[k] = sm + elems + t + k * A.nd * T;
+			step[k] = T;
+			if (GLOBAL && k >= A.nsm) {
+				own[k] = (k < 4 ? A.scratch[k] + (size_t)unit * A.npts : x) + B.go;
+				step[k] = B.s3;
+			}
+		}
+		auto at = [&](int k, int d) -> double & { return own[k][d * step[k]]; };
 		for (int e = t; e < elems; e += T) sm[e] = 0.0;
 		__syncthreads();
 		double r[D], u[D], w[D];
@@ -892,8 +908,8 @@ __global__ void __launch_bounds__(512, 1) k_res_pcg(const __grid_constant__ ResA
 			B.residual<D, UNIT>(A, x, A.rhs + (size_t)unit * A.npts, [&](int d, double xi, double bi, double ri) {
 				r[d] = ri;
 				u[d] = mul(ri, im);  // :138
-				fx[d * T] = xi;
-				fq[d * T] = fs[d * T] = fp[d * T] = fz[d * T] = 0.0;  // :146-149
+				at(4, d) = xi;
+				at(0, d) = at(1, d) = at(2, d) = at(3, d) = 0.0;  // :146-149
 				sm[B.so + d * B.pp] = u[d];
 				B.publish(A, faces, d, u[d]);
 				v[0] = fma(bi, bi, v[0]);
@@ -951,16 +967,17 @@ __global__ void __launch_bounds__(512, 1) k_res_pcg(const __grid_constant__ ResA
 				const double alpha = st.alpha, beta = st.beta;
 				v[0] = v[1] = v[2] = 0.0;
 				B.march<D, UNIT, false>(A, sm, 1.0, [&](int d, double mi, double ni) {  // n = A m (:161-184)
-					const double qi = add(mi, mul(beta, fq[d * T]));      // :200
-					const double si = add(w[d], mul(beta, fs[d * T]));    // :203
-					const double pi = add(u[d], mul(beta, fp[d * T]));    // :206
-					const double zi = add(ni, mul(beta, fz[d * T]));      // :209
-					fq[d * T] = qi;
-					fs[d * T] = si;
-					fp[d * T] = pi;
-					fz[d * T] = zi;
+					const double qi = add(mi, mul(beta, at(0, d)));       // :200
+					const double si = add(w[d], mul(beta, at(1, d)));     // :203
+					const double pi = add(u[d], mul(beta, at(2, d)));     // :206
+					const double zi = add(ni, mul(beta, at(3, d)));       // :209
+					const double xi = add(at(4, d), mul(alpha, pi));      // :215
+					at(0, d) = qi;
+					at(1, d) = si;
+					at(2, d) = pi;
+					at(3, d) = zi;
+					at(4, d) = xi;
 					r[d] = add(r[d], mul(-alpha, si));                    // :212
-					fx[d * T] = add(fx[d * T], mul(alpha, pi));           // :215
 					u[d] = add(u[d], mul(-alpha, qi));                    // :218
 					w[d] = add(w[d], mul(-alpha, zi));                    // :221
 					B.publish(A, out, d, mul(w[d], im));
@@ -981,8 +998,8 @@ __global__ void __launch_bounds__(512, 1) k_res_pcg(const __grid_constant__ ResA
 				    }))
 					return;
 			}
-			if (B.own)
-				for (int d = 0; d < B.nd; d++) stl2(x + B.go + d * B.s3, fx[d * T]);
+			if (B.own && (!GLOBAL || A.nsm > 4))
+				for (int d = 0; d < B.nd; d++) stl2(x + B.go + d * B.s3, at(4, d));
 		}
 		if (blockIdx.x % A.G == 0 && t == 0) write_state(st, A, unit);
 		__syncthreads();  // shared memory is reused by the next right-hand side
@@ -995,10 +1012,10 @@ __global__ void __launch_bounds__(512, 1) k_res_pcg(const __grid_constant__ ResA
 // registers.  Three group reductions an iteration; the first publishes the
 // boundary rows of v, the third those of r, and every block forms its ghosts
 // of p and s from them (times iM at each read, as the reference rounds p_hat
-// and s_hat).
+// and s_hat).  Boxes of more than 8 planes leave x in global memory (A.nsm 1).
 // ---------------------------------------------------------------------------
-template <int D, bool UNIT>
-__global__ void __launch_bounds__(512, 1) k_res_bicg(const __grid_constant__ ResArgs A) {
+template <int D, int TMAX, bool UNIT>
+__global__ void __launch_bounds__(TMAX, 1) k_res_bicg(const __grid_constant__ ResArgs A) {
 	extern __shared__ __align__(16) unsigned char smem[];
 	__shared__ ResGroup gsh;
 	__shared__ KrylovState st;
@@ -1007,7 +1024,8 @@ __global__ void __launch_bounds__(512, 1) k_res_bicg(const __grid_constant__ Res
 	const int t = threadIdx.x, T = blockDim.x;
 	const int elems = B.pp * (A.nd + 2) + 1;
 	double *const sp = reinterpret_cast<double *>(smem), *const ss = sp + elems;
-	double *const fx = ss + elems + t, *const fh = fx + A.nd * T;  // own x, r_hat of plane d at [d * T]
+	constexpr bool GLOBAL = D > 8;
+	double *const fh = ss + elems + t;  // own r_hat of plane d at [d * T]
 	double *const rfaces = static_cast<double *>(A.edge) + (size_t)blockIdx.x * B.face_rows * A.n1;
 	// v's faces of two iterations: a block publishes new rows while a neighbour
 	// may still form its p from the old ones.
@@ -1026,6 +1044,9 @@ __global__ void __launch_bounds__(512, 1) k_res_bicg(const __grid_constant__ Res
 	for (int unit = blockIdx.x / A.G; unit < A.lanes; unit += A.groups) {
 		double *const x = A.x + (size_t)unit * A.npts;
 		const bool hist = A.hist && unit == 0 && blockIdx.x % A.G == 0;
+		const bool xg = GLOBAL && A.nsm < 2;
+		double *const fx = xg ? x + B.go : fh + A.nd * T;  // own x of plane d at [d * xstep]
+		const int xstep = xg ? B.s3 : T;
 		for (int e = t; e < 2 * elems; e += T) sp[e] = 0.0;
 		__syncthreads();
 		double r[D], vv[D], tt[D];
@@ -1033,7 +1054,7 @@ __global__ void __launch_bounds__(512, 1) k_res_bicg(const __grid_constant__ Res
 			double v[2] = {0.0, 0.0};
 			B.residual<D, UNIT>(A, x, A.rhs + (size_t)unit * A.npts, [&](int d, double xi, double bi, double ri) {
 				r[d] = ri;
-				fx[d * T] = xi;
+				fx[d * xstep] = xi;
 				fh[d * T] = ri;  // r_hat = r (:153)
 				B.publish(A, rfaces, d, ri);
 				v[0] = fma(bi, bi, v[0]);
@@ -1112,12 +1133,12 @@ __global__ void __launch_bounds__(512, 1) k_res_bicg(const __grid_constant__ Res
 				for (int d = 0; d < D; d++) {
 					if (d >= B.nd) break;
 					const double ph = mul(sp[B.so + d * B.pp], im), si = ss[B.so + d * B.pp];
-					const double x1 = add(fx[d * T], mul(alpha, ph));
+					const double x1 = add(fx[d * xstep], mul(alpha, ph));
 					if (s_exit) {
-						fx[d * T] = x1;  // :196
+						fx[d * xstep] = x1;  // :196
 						continue;
 					}
-					fx[d * T] = add(x1, mul(omega, mul(si, im)));  // :216
+					fx[d * xstep] = add(x1, mul(omega, mul(si, im)));  // :216
 					r[d] = add(si, mul(-omega, tt[d]));            // :219
 					B.publish(A, rfaces, d, r[d]);
 					v[0] = fma(r[d], r[d], v[0]);
@@ -1150,8 +1171,8 @@ __global__ void __launch_bounds__(512, 1) k_res_bicg(const __grid_constant__ Res
 			    }))
 				return;
 		}
-		if (st.reason != STOP_EARLY && B.own)
-			for (int d = 0; d < B.nd; d++) stl2(x + B.go + d * B.s3, fx[d * T]);
+		if (st.reason != STOP_EARLY && B.own && !xg)
+			for (int d = 0; d < B.nd; d++) stl2(x + B.go + d * B.s3, fx[d * xstep]);
 		if (blockIdx.x % A.G == 0 && t == 0) write_state(st, A, unit);
 		__syncthreads();  // shared memory is reused by the next right-hand side
 	}
@@ -1169,12 +1190,13 @@ typedef void (*ResKernel)(const ResArgs);
 // Box shapes: C rows x at most D planes per thread, at most T threads, so many
 // blocks per SM.  The last ones, one row per thread, are those of pipelined CG
 // and BiCGStab.
-constexpr int kShapes = 9, kCgShapes = 6;
-constexpr int kShapeC[kShapes] = {1, 1, 2, 2, 3, 2, 1, 1, 1}, kShapeD[kShapes] = {2, 8, 8, 16, 16, 16, 2, 4, 8},
-              kShapeT[kShapes] = {512, 512, 512, 512, 384, 256, 512, 512, 512},
-              kShapeB[kShapes] = {1, 1, 1, 1, 1, 2, 1, 1, 1};
-// Fields of a solver in shared memory with ghosts, and own points only; fields
-// whose faces it publishes.
+constexpr int kShapes = 10, kCgShapes = 6;
+constexpr int kShapeC[kShapes] = {1, 1, 2, 2, 3, 2, 1, 1, 1, 1}, kShapeD[kShapes] = {2, 8, 8, 16, 16, 16, 2, 4, 8, 16},
+              kShapeT[kShapes] = {512, 512, 512, 512, 384, 256, 512, 512, 512, 384},
+              kShapeB[kShapes] = {1, 1, 1, 1, 1, 2, 1, 1, 1, 1};
+// Fields of a solver in shared memory with ghosts, and own points only (of
+// which the last shape may leave some in global memory); fields whose faces
+// it publishes.
 constexpr int kGhosted[4] = {0, 2, 1, 1}, kOwn[4] = {0, 2, 0, 5}, kFaces[4] = {0, 3, 1, 2};  // by solver id
 
 template <class V, bool UNIT>
@@ -1192,9 +1214,10 @@ ResKernel cg_kernel(int shape) {
 template <bool UNIT>
 ResKernel krylov_kernel(int ks, int shape) {
 	switch (shape) {
-	case 6: return ks == SEDI_BICGSTAB ? (ResKernel)k_res_bicg<2, UNIT> : (ResKernel)k_res_pcg<2, UNIT>;
-	case 7: return ks == SEDI_BICGSTAB ? (ResKernel)k_res_bicg<4, UNIT> : (ResKernel)k_res_pcg<4, UNIT>;
-	default: return ks == SEDI_BICGSTAB ? (ResKernel)k_res_bicg<8, UNIT> : (ResKernel)k_res_pcg<8, UNIT>;
+	case 6: return ks == SEDI_BICGSTAB ? (ResKernel)k_res_bicg<2, 512, UNIT> : (ResKernel)k_res_pcg<2, 512, UNIT>;
+	case 7: return ks == SEDI_BICGSTAB ? (ResKernel)k_res_bicg<4, 512, UNIT> : (ResKernel)k_res_pcg<4, 512, UNIT>;
+	case 8: return ks == SEDI_BICGSTAB ? (ResKernel)k_res_bicg<8, 512, UNIT> : (ResKernel)k_res_pcg<8, 512, UNIT>;
+	default: return ks == SEDI_BICGSTAB ? (ResKernel)k_res_bicg<16, 384, UNIT> : (ResKernel)k_res_pcg<16, 384, UNIT>;
 	}
 }
 
@@ -1205,7 +1228,7 @@ ResKernel kernel_for(int ks, bool fp32, bool unit, int shape) {
 }
 
 struct Plan {
-	int shape = -1, G = 0, groups = 0, RG = 0, T = 0, s2 = 0, nd = 0;
+	int shape = -1, G = 0, groups = 0, RG = 0, T = 0, s2 = 0, nd = 0, nsm = 0;
 	size_t smem = 0;
 };
 
@@ -1216,7 +1239,8 @@ struct Plan {
 // 20100), 1.65 with two stencil passes (16384: 38000), 1.8 at three rows a
 // thread (12672: 32500), and 3.2 with two blocks on an SM (2 x 8192: 37400).
 // Pipelined CG: 256 points a block 7700, 2048 10400, 4096 14000; BiCGStab: 512
-// points 19000, 2048 24000, 4096 29000.
+// points 19000, 2048 24000, 4096 29000, 6144 (x in L2) 52000; pipelined CG's
+// 6144 points (two or three fields in L2) 27700.
 Plan plan_for(int ks, const Geo &g, int units, int sms, size_t smem_max, double *cycles) {
 	constexpr double kPoint[kCgShapes] = {1.3, 1.3, 1.3, 1.65, 1.8, 3.2};
 	constexpr double kSync[4] = {0.0, 16000.0, 9000.0, 6000.0}, kPointOf[4] = {0.0, 2.9, 0.0, 1.6};  // by solver id
@@ -1228,12 +1252,17 @@ Plan plan_for(int ks, const Geo &g, int units, int sms, size_t smem_max, double 
 			const int T = (RG * g.n1 + 31) / 32 * 32, B2 = RG * C, s2 = (g.n2 + B2 - 1) / B2;
 			for (int nd = 1; nd <= kShapeD[sh] && nd <= g.n3; nd++) {
 				const long long G = (long long)s2 * ((g.n3 + nd - 1) / nd);
-				const size_t smem = (((size_t)(g.n1 + 1) * (B2 + 2) * (nd + 2) + 1) * kGhosted[ks] + (size_t)kOwn[ks] * nd * T) * 8;
+				const size_t ghosted = ((size_t)(g.n1 + 1) * (B2 + 2) * (nd + 2) + 1) * kGhosted[ks] * 8, own = (size_t)nd * T * 8;
+				int nsm = kOwn[ks];
+				if (sh == kShapes - 1)
+					while (nsm > (ks == SEDI_BICGSTAB ? 1 : 0) && ghosted + nsm * own > smem_max) nsm--;
+				const size_t smem = ghosted + nsm * own;
 				if (G > slots || smem * kShapeB[sh] > smem_max) continue;
 				const int groups = units < slots / (int)G ? units : slots / (int)G;
-				const double point = ks == SEDI_CG ? kPoint[sh < kCgShapes ? sh : 0] : kPointOf[ks];
-				const double deep = ks != SEDI_CG && nd > 4 ? 1500.0 : 0.0;  // the 8-plane kernels' start-up
-				const double cost = ((G > 1 ? kSync[ks] + 15.0 * G : kSync[ks] / 3.0) + deep + point * T * C * nd) *
+				const double point = ks == SEDI_CG ? kPoint[sh < kCgShapes ? sh : 0] : kPointOf[ks] * (ks == SEDI_BICGSTAB && nd > 8 ? 1.7 : 1.0);
+				const double deep = ks != SEDI_CG && nd > 4 ? 1500.0 : 0.0;  // the deeper kernels' start-up
+				const double cost = ((G > 1 ? kSync[ks] + 15.0 * G : kSync[ks] / 3.0) + deep +
+				                     (point + 0.75 * (kOwn[ks] - nsm)) * T * C * nd) *
 				                    ((units + groups - 1) / groups);
 				if (best.shape >= 0 && cost >= *cycles) continue;
 				*cycles = cost;
@@ -1244,6 +1273,7 @@ Plan plan_for(int ks, const Geo &g, int units, int sms, size_t smem_max, double 
 				best.T = T;
 				best.s2 = s2;
 				best.nd = nd;
+				best.nsm = nsm;
 				best.smem = smem;
 			}
 		}
@@ -1391,6 +1421,8 @@ int resident_launch(Ctx *c, Resident *R, const ResIO &io) {
 	a.s2 = p.s2;
 	a.RG = p.RG;
 	a.nd = p.nd;
+	a.nsm = p.nsm;
+	for (int k = 0; k < 4; k++) a.scratch[k] = io.scratch[k];
 	a.rhs = io.rhs;
 	a.x = io.x;
 	a.xlo = (float2 *)io.xlo;

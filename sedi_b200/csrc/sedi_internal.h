@@ -149,6 +149,7 @@ struct ResIO {
 	const double *rhs;
 	double *x;             // FP64: x; FP32: x_hi
 	void *xlo;             // FP32: scratch of one Krylov field
+	double *scratch[4];    // pipelined CG: scratch of q, s, p, z
 	double tol, tol_in;
 	int maxiter, period;
 	double *o_err, *o_bb, *o_rr;  // device, per right-hand side

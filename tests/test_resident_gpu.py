@@ -20,7 +20,7 @@ pytestmark = pytest.mark.gpu
 # block row (512), one point wide, every box shape's size range, and the first
 # grid that is too wide (513).
 @pytest.mark.parametrize("dims", [(33, 17, 9), (97, 65, 51), (128, 33, 70), (512, 6, 5), (513, 4, 3), (1, 40, 37),
-                                  (31, 1, 64), (64, 64, 64), (300, 40, 30), (100, 110, 120), (80, 85, 88)])
+                                  (31, 1, 64), (64, 64, 64), (300, 40, 30), (100, 110, 120), (80, 85, 88), (96, 96, 96), (61, 100, 131)])
 @pytest.mark.parametrize("coeffs", [(6.0, 1.0, 1.0), (6.5, 1.2, 0.9)])
 @pytest.mark.parametrize("solver,K", [("cg", 21), ("pcg", 21), ("bicgstab", 12)])
 def test_single_vector_matches_oracle(dims, coeffs, solver, K):
