@@ -505,7 +505,14 @@ struct OpBase {
 	__device__ void gload(long long, Vec<T> *) const {}
 	__device__ bool enabled(const Global *) const { return true; }
 	__device__ void after(Global *) const {}  // last block, after every lane's fin
-	__device__ bool slice_live(const Global *, const LaneState &, int, int) const { return true; }
+	// A block whose lanes have all finished (padding lanes from the start) streams
+	// nothing and only joins the reduction: 40 mixed right-hand sides pad to 64
+	// lanes, and a batch's lanes converge at different iterations.
+	__device__ bool slice_live(const Global *, const LaneState &ls, int lane0, int nl) const {
+		for (int l = lane0; l < lane0 + nl; l++)
+			if (!ls.done[l]) return true;
+		return false;
+	}
 };
 
 // ---------------------------------------------------------------------------
@@ -531,9 +538,9 @@ struct OpResid : OpBase<double> {
 	__device__ bool enabled(const Global *gl) const { return !ru || gl->ru_due; }
 	// A reliable update triggered by single lanes sweeps only their slices.
 	__device__ bool slice_live(const Global *gl, const LaneState &ls, int lane0, int nl) const {
-		if (!ru || pcg || gl->ru_all) return true;
+		if (!ru) return true;
 		for (int l = lane0; l < lane0 + nl; l++)
-			if (ls.pending[l]) return true;
+			if (!ls.done[l] && (pcg || gl->ru_all || ls.pending[l])) return true;
 		return false;
 	}
 	__device__ bool raw_center() const { return false; }
@@ -781,6 +788,12 @@ struct OpCgB : OpBase<T> {
 	// iteration, so the other sees b_iter != iter and leaves.
 	__device__ bool enabled(const Global *gl) const {
 		return XS == XS_EVERY || (gl->b_iter == gl->iter && (gl->iter & 1) == (XS == XS_R ? 1 : 0));
+	}
+	// A lane that stopped in the odd form still takes its deferred step here.
+	__device__ bool slice_live(const Global *, const LaneState &ls, int lane0, int nl) const {
+		for (int l = lane0; l < lane0 + nl; l++)
+			if (!ls.done[l] || (XS == XS_X && ls.xa[l] != 0.0)) return true;
+		return false;
 	}
 	__device__ void after(Global *gl) const {
 		if (XS != XS_EVERY) gl->x_pending = XS == XS_R ? 1 : 0;
@@ -1349,7 +1362,7 @@ __global__ void kb_ru_done(Global *gl) {
 __global__ void __launch_bounds__(256) kb_ru_fold(long long npts, int R, int WD, int WT, double *__restrict__ xh,
                                                   float *__restrict__ xl, const float *__restrict__ p_odd,
                                                   const double *__restrict__ xa, const int *__restrict__ pending,
-                                                  int all, Global *gl) {
+                                                  const int *__restrict__ done, int all, Global *gl) {
 	if (gl->active == 0 || gl->ru_due == 0) return;
 	all = all || gl->ru_all;
 	const bool step = p_odd != nullptr && (gl->iter & 1);
@@ -1361,7 +1374,8 @@ __global__ void __launch_bounds__(256) kb_ru_fold(long long npts, int R, int WD,
 		const long long rem = od - sd * WD * npts;
 		const long long i = rem / WD;
 		const int j = (int)(sd * WD + rem % WD);
-		const bool f0 = all || pending[j], f1 = all || pending[j + 1];  // lanes j, j+1 share the pair
+		// Lanes j, j+1 share the pair; a finished lane's x_lo is zero.
+		const bool f0 = !done[j] && (all || pending[j]), f1 = !done[j + 1] && (all || pending[j + 1]);
 		if (!f0 && !f1) continue;
 		// Both lanes of the pair fold x_lo (x_hi + x_lo is unchanged for a
 		// lane outside the update); only the lanes in the update take their
@@ -2150,7 +2164,7 @@ static void enqueue_cg_iteration(Ctx *c, Batched *B) {
 		const long long nb = ((long long)B->elems / 2 + 255) / 256;
 		kb_ru_fold<<<(int)(nb < 148 * 16 ? nb : 148 * 16), 256, 0, s>>>(c->g.n, B->R, B->rbD, B->rbT, B->xh,
 		                                                                 (float *)B->x, B->defer_x ? (const float *)B->p1 : nullptr,
-		                                                                 B->ls.xa, B->ls.pending, B->ks == 3 ? 1 : 0, B->gl);
+		                                                                 B->ls.xa, B->ls.pending, B->ls.done, B->ks == 3 ? 1 : 0, B->gl);
 		c->launches++;
 		enqueue_resid<RBD, PAIRS>(c, B, true);
 		kb_ru_done<<<1, 1, 0, s>>>(B->gl);
@@ -2203,7 +2217,7 @@ static void enqueue_pcg_iteration(Ctx *c, Batched *B) {
 		const long long nb = ((long long)B->elems / 2 + 255) / 256;
 		kb_ru_fold<<<(int)(nb < 148 * 16 ? nb : 148 * 16), 256, 0, s>>>(c->g.n, B->R, B->rbD, B->rbT, B->xh,
 		                                                                 (float *)B->x, nullptr, B->ls.xa, B->ls.pending,
-		                                                                 B->ks == 3 ? 1 : 0, B->gl);
+		                                                                 B->ls.done, B->ks == 3 ? 1 : 0, B->gl);
 		c->launches++;
 		enqueue_resid<RBD, PAIRS>(c, B, true);
 		OpApply<T> a1;
@@ -2291,7 +2305,7 @@ static void enqueue_bicg_iteration(Ctx *c, Batched *B) {
 		const long long nb = ((long long)B->elems / 2 + 255) / 256;
 		kb_ru_fold<<<(int)(nb < 148 * 16 ? nb : 148 * 16), 256, 0, s>>>(c->g.n, B->R, B->rbD, B->rbT, B->xh,
 		                                                                 (float *)B->x, nullptr, B->ls.xa, B->ls.pending,
-		                                                                 B->ks == 3 ? 1 : 0, B->gl);
+		                                                                 B->ls.done, B->ks == 3 ? 1 : 0, B->gl);
 		c->launches++;
 		enqueue_resid<RBD, PAIRS>(c, B, true);
 		kb_ru_done<<<1, 1, 0, s>>>(B->gl);
