@@ -148,6 +148,7 @@ __global__ void __launch_bounds__(C::THREADS, C::MINB) k_stream(SGeo g, const __
 	              NPS = C::NPS, KC = C::KC, KO = C::KO, ME = C::ME;
 	constexpr int NS = Op::NS, NQ = Op::NQ, ND = Op::ND, NGX = Op::NG > 0 ? Op::NG : 1;
 	constexpr bool IDENT = Op::IDENT, INPLACE = Op::INPLACE, STAGED = IDENT || INPLACE;
+	constexpr bool DOWN = Op::DOWN;  // planes from z1 to z0-1 instead of z0-1 to z1
 	typedef Layout<C, NS, NQ, ND, IDENT, INPLACE> Lay;
 	constexpr int NST = Lay::NST, KEEP = Lay::KEEP;
 	extern __shared__ __align__(128) unsigned char smem[];
@@ -214,8 +215,9 @@ __global__ void __launch_bounds__(C::THREADS, C::MINB) k_stream(SGeo g, const __
 	}
 	__syncthreads();
 
+	auto plane_of = [&](int j) { return DOWN ? z1 - j : z0 - 1 + j; };  // grid plane of step j
 	auto issue = [&](int j) {  // thread 0
-		const int p = z0 - 1 + j;
+		const int p = plane_of(j);
 		uint64_t *b = &bar[j % NST];
 		E *st = stage0 + (j % NST) * SE;
 		if (p < 0 || p >= g.n3) {
@@ -232,8 +234,8 @@ __global__ void __launch_bounds__(C::THREADS, C::MINB) k_stream(SGeo g, const __
 #pragma unroll
 		for (int q = 0; q < NQ; q++) tma_load3(st + NS * HE + q * IE, &maps.m[op.q_map(q)], b, i1_0 * ME, i2_0, zoff + p);
 		// The same tiles pfd planes further on, into L2 (within this block's planes).
-		const int pf = p + g.pfd;
-		if (g.pfd > 0 && pf <= z1 && pf < g.n3) {
+		const int pf = DOWN ? p - g.pfd : p + g.pfd;
+		if (g.pfd > 0 && (DOWN ? pf >= z0 - 1 && pf >= 0 : pf <= z1 && pf < g.n3)) {
 #pragma unroll
 			for (int s = 0; s < NS; s++) tma_prefetch3(&maps.m[op.src_map(s)], (i1_0 - 1) * ME, i2_0 - 1, zoff + pf);
 #pragma unroll
@@ -266,14 +268,14 @@ __global__ void __launch_bounds__(C::THREADS, C::MINB) k_stream(SGeo g, const __
 		// transform, so they are in flight during it.
 		Vec<T> gv[KO][NGX];
 		if (Op::NG > 0 && j >= 3) {
-			const long long zb = (long long)(z0 - 1 + j - 2) * plane;
+			const long long zb = (long long)plane_of(j - 2) * plane;
 #pragma unroll
 			for (int k = 0; k < KO; k++)
 				if (oval >> k & 1u) op.gload(((long long)slice * g.npts + zb + obase[k]) * RB + lo, gv[k]);
 		}
 		// Phase 1: stencil input of plane j (transforming ops only).
 		if (!IDENT && j < np) {
-			const int p = z0 - 1 + j;
+			const int p = plane_of(j);
 			E *const st = stage0 + sj * SE;
 			// In place: over the source field INPLACE_SLOT of this plane's stage
 			// (each thread rewrites only the points it read).
@@ -300,7 +302,7 @@ __global__ void __launch_bounds__(C::THREADS, C::MINB) k_stream(SGeo g, const __
 		// Phase 2: outputs of plane m = j-2 from planes m-1, m, m+1.
 		if (j >= 3) {
 			const int m = j - 2;
-			const int z = z0 - 1 + m;
+			const int z = plane_of(m);
 			// Stage slots of planes m-1, m, m+1 (sj is the slot of plane j = m+2).
 			const int sm1 = sj >= 3 ? sj - 3 : sj - 3 + NST;
 			const int s0 = sj >= 2 ? sj - 2 : sj - 2 + NST;
@@ -313,8 +315,8 @@ __global__ void __launch_bounds__(C::THREADS, C::MINB) k_stream(SGeo g, const __
 				cm = stage0 + sm1 * SE + off;
 				c0 = stz + off;
 				cp = stage0 + sp1 * SE + off;
-				zm = z - 1 >= 0;
-				zp = z + 1 < g.n3;
+				zm = DOWN ? z + 1 < g.n3 : z - 1 >= 0;
+				zp = DOWN ? z - 1 >= 0 : z + 1 < g.n3;
 			} else {
 				cm = ring + ((m - 1) & 3) * HE;
 				c0 = ring + (m & 3) * HE;
@@ -341,8 +343,8 @@ __global__ void __launch_bounds__(C::THREADS, C::MINB) k_stream(SGeo g, const __
 				const Vec<T> xp1 = lds(c0 + hc + RB);
 				const Vec<T> xm2 = (ROWS && k > 0) ? zcur[k > 0 ? k - 1 : 0] : lds(c0 + hc - H1 * RB);
 				const Vec<T> xp2 = (ROWS && k + 1 < KO) ? zcur[k + 1 < KO ? k + 1 : k] : lds(c0 + hc + H1 * RB);
-				const Vec<T> &xm3 = zprev[k];
-				const Vec<T> &xp3 = znext[k];
+				const Vec<T> &xm3 = DOWN ? znext[k] : zprev[k];
+				const Vec<T> &xp3 = DOWN ? zprev[k] : znext[k];
 				Vec<T> y;
 				if constexpr (Op::SCALED) {
 					// The ring holds f and the stencil input is f .* iM: FP64
@@ -495,6 +497,9 @@ struct OpBase {
 	static constexpr int NG = 0;    // pointwise fields read with plain loads, prefetched by gload
 	static constexpr bool INPLACE = false;  // stencil input written over source INPLACE_SLOT (no ring)
 	static constexpr int INPLACE_SLOT = 1;
+	// DOWN: the sweep runs the planes downwards, so that it starts with what the
+	// upward sweep before it left in L2, and leaves what the next one starts with.
+	static constexpr bool DOWN = false;
 	// SCALED: src() gives f and the stencil is applied to f .* iMc (the op
 	// provides iMc and, for FP32, the scaled coefficients kas, kbs, kcs).
 	static constexpr bool SCALED = false;
@@ -776,7 +781,7 @@ struct OpCgB : OpBase<T> {
 	// XS_R streams two words like sweep A and takes its 32x32 tiles (KIND 1).
 	static constexpr int KIND = XS == XS_R ? 1 : 0;
 	static constexpr int NS = 1, NQ = XS == XS_EVERY ? 2 : (XS == XS_R ? 1 : 3), ND = 2;
-	static constexpr bool IDENT = true, USES_RAW_CENTER = false, ADVANCE = true;
+	static constexpr bool IDENT = true, USES_RAW_CENTER = false, ADVANCE = true, DOWN = true;
 	static constexpr int V = Vec<T>::V;
 	T iMc;
 	T *x, *r;
