@@ -549,6 +549,12 @@ struct OpResid : OpBase<double> {
 		return false;
 	}
 	__device__ bool raw_center() const { return false; }
+	// The update ends the iteration (pipelined CG's own sweeps still follow).
+	__device__ void after(Global *gl) const {
+		if (!ru || pcg) return;
+		gl->ru_due = gl->ru_all = 0;
+		gl->iter += 1;
+	}
 	__device__ void begin(const Global *gl, const LaneState &ls, int lane) {
 		it = gl->iter;
 		for (int e = 0; e < 2; e++) {
@@ -2138,8 +2144,11 @@ static OpCgB<T, XS> cg_b_as(const OpCgB<T> &o) {
 	return d;
 }
 
+// parity: of the iteration's number, or -1 where the captured graph does not
+// fix it (both parity forms of sweep B are captured and one leaves at once, 3
+// to 5 us).
 template <class T, int RBT, int RBD, bool PAIRS = false>
-static void enqueue_cg_iteration(Ctx *c, Batched *B) {
+static void enqueue_cg_iteration(Ctx *c, Batched *B, int parity) {
 	cudaStream_t s = c->stream;
 	OpCgA<T> a;
 	a.ka = (T)c->k.a;
@@ -2159,9 +2168,8 @@ static void enqueue_cg_iteration(Ctx *c, Batched *B) {
 	bo.r = (T *)B->r;
 	bo.mixed = B->mixed ? 1 : 0;
 	if (B->defer_x) {
-		// Both are captured; each runs only on its iteration parity.
-		launchT<T, RBT, PAIRS>(c, B, cg_b_as<XS_R>(bo), s);
-		launchT<T, RBT, PAIRS>(c, B, cg_b_as<XS_X>(bo), s);
+		if (parity != 0) launchT<T, RBT, PAIRS>(c, B, cg_b_as<XS_R>(bo), s);
+		if (parity != 1) launchT<T, RBT, PAIRS>(c, B, cg_b_as<XS_X>(bo), s);
 	} else {
 		launchT<T, RBT, PAIRS>(c, B, bo, s);
 	}
@@ -2172,8 +2180,6 @@ static void enqueue_cg_iteration(Ctx *c, Batched *B) {
 		                                                                 B->ls.xa, B->ls.pending, B->ls.done, B->ks == 3 ? 1 : 0, B->gl);
 		c->launches++;
 		enqueue_resid<RBD, PAIRS>(c, B, true);
-		kb_ru_done<<<1, 1, 0, s>>>(B->gl);
-		c->launches++;
 	}
 }
 
@@ -2313,8 +2319,6 @@ static void enqueue_bicg_iteration(Ctx *c, Batched *B) {
 		                                                                 B->ls.done, B->ks == 3 ? 1 : 0, B->gl);
 		c->launches++;
 		enqueue_resid<RBD, PAIRS>(c, B, true);
-		kb_ru_done<<<1, 1, 0, s>>>(B->gl);
-		c->launches++;
 	}
 }
 
@@ -2355,7 +2359,7 @@ struct Impl {
 			for (int i = 0; i < B->chunk; i++) {
 				if (B->ks == 3) enqueue_pcg_iteration<T, RBT, RBD, PAIRS>(c, B);
 				else if (B->ks == 1) enqueue_bicg_iteration<T, RBT, RBD, PAIRS>(c, B);
-				else enqueue_cg_iteration<T, RBT, RBD, PAIRS>(c, B);
+				else enqueue_cg_iteration<T, RBT, RBD, PAIRS>(c, B, B->chunk % 2 == 0 ? (i + 1) & 1 : -1);
 			}
 			if (B->defer_x && !B->mixed) {  // the mixed form folds pending steps in its reliable update
 				const long long npts = PAIRS ? c->g.n / 2 : c->g.n;
