@@ -234,6 +234,10 @@ typedef struct sedi_slab_args {
  */
 int sedi_slab_sweep(int mode, long n1, long n2, long nloc, double a, double b, double c, long z_lo, long z_hi,
                     const sedi_slab_args *args, double *chunk_part, double *plane_part, void *stream);
+/* The three dot products of a sweep: plane_part's n3 rows summed in an order
+ * fixed by n3, into host memory (best pinned), by way of scratch (3 doubles,
+ * device).  Waits for the stream. */
+int sedi_slab_totals(long n3, const double *plane_part, double *scratch, double *totals, void *stream);
 /* t += x .* v, q += v .* v (t = x .* v, q = v .* v when reset) over n elements
  * (stochastic-estimator.cc:195, :198). */
 int sedi_slab_accumulate(long n, const double *x, const double *v, double *t, double *q, int reset, void *stream);

@@ -27,7 +27,10 @@ namespace sedi {
 namespace {
 
 constexpr int kSlabThreads = 256;
-constexpr int kSlabChunks = 8;  // row chunks per plane (fixed: the summation order depends on it)
+// Row chunks per plane, a block each (fixed: the summation order depends on
+// it).  A block's rows are a serial chain of loads: with 8 chunks a slab of
+// 192 x 160 x 64 gave 512 blocks of 20 rows, 43% of the warps an SM holds.
+constexpr int kSlabChunks = 32;
 constexpr int kSlabDots = 3;    // dot products per plane
 
 struct SlabGeo {
@@ -62,6 +65,7 @@ __device__ __forceinline__ double slab_stencil(const SlabGeo &g, const Coef &k, 
 template <int ND>
 __device__ __forceinline__ void block_total(double (&v)[ND]) {
 	__shared__ double sh[kSlabThreads / 32][ND];
+	const int nw = blockDim.x >> 5;
 	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 	warp_sum<ND>(v);
 	if (lane == 0)
@@ -72,12 +76,18 @@ __device__ __forceinline__ void block_total(double (&v)[ND]) {
 #pragma unroll
 		for (int d = 0; d < ND; d++) {
 			double s = 0.0;
-			for (int w = 0; w < kSlabThreads / 32; w++) s += sh[w][d];
+			for (int w = 0; w < nw; w++) s += sh[w][d];
 			v[d] = s;
 		}
 	}
 	__syncthreads();
 }
+
+// Threads of a row: whole warps covering n1, at most the block.  A block is as
+// many such rows as fit it, so that no warp idles (n1 = 192: blocks of 192
+// threads; rounding to a power of two left a quarter of 256 idle).
+__host__ __device__ __forceinline__ int row_threads(int n1) { return n1 >= kSlabThreads ? kSlabThreads : (n1 + 31) / 32 * 32; }
+__host__ __device__ __forceinline__ int block_threads(int n1) { return kSlabThreads / row_threads(n1) * row_threads(n1); }
 
 enum SlabMode {
 	SLAB_SETUP = 0,       // r = b - A src; <b,b>, <r,r>                          (Cg.hpp:112-129)
@@ -121,14 +131,11 @@ __global__ void __launch_bounds__(kSlabThreads) k_slab_sweep(SlabGeo g, Coef k, 
 #pragma unroll
 	for (int d = 0; d < ND; d++) v[d] = 0.0;
 	const double iM = a.iM;
-	// Rows of the chunk, each by tpr threads (the smallest power of two >= n1,
-	// at most the block), the block's other threads on the next rows.  Not
-	// unrolled: these sweeps hide latency with resident warps, and unrolling
-	// by 4 cost more in occupancy (registers) than it gained (512^3 CG 55 ->
-	// 51, pipelined CG 46 -> 37 GPoint-it/s on B200).
-	int tpr = 32;
-	while (tpr < g.n1 && tpr < kSlabThreads) tpr <<= 1;
-	const int rpi = kSlabThreads / tpr, tc = (int)threadIdx.x % tpr;
+	// Rows of the chunk, each by tpr threads (row_threads), the block's other
+	// threads on the next rows.  Not unrolled: these sweeps hide latency with
+	// resident warps, and unrolling by 4 cost more in occupancy (registers) than
+	// it gained (512^3 CG 55 -> 51, pipelined CG 46 -> 37 GPoint-it/s on B200).
+	const int tpr = row_threads(g.n1), rpi = blockDim.x / tpr, tc = (int)threadIdx.x % tpr;
 	for (int i1 = tc; i1 < g.n1; i1 += tpr) {
 #pragma unroll 1
 		for (int i2 = r0 + (int)threadIdx.x / tpr; i2 < r1; i2 += rpi) {
@@ -228,15 +235,28 @@ __global__ void __launch_bounds__(kSlabThreads) k_slab_sweep(SlabGeo g, Coef k, 
 	}
 }
 
-// Per-plane sums of the chunk partials, chunks in order.
-__global__ void k_slab_plane_sums(int z_lo, int z_hi, const double *chunk_part, double *plane_part) {
-	const int z = z_lo + blockIdx.x * blockDim.x + threadIdx.x;
+// Per-plane sums of the chunk partials in a fixed tree: a warp per plane, a
+// lane per chunk.
+__global__ void __launch_bounds__(128) k_slab_plane_sums(int z_lo, int z_hi, const double *chunk_part, double *plane_part) {
+	static_assert(kSlabChunks == 32, "a lane per chunk");
+	const int z = z_lo + (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
 	if (z >= z_hi) return;
-	for (int d = 0; d < kSlabDots; d++) {
-		double s = 0.0;
-		for (int c = 0; c < kSlabChunks; c++) s += chunk_part[((size_t)(z - 1) * kSlabChunks + c) * kSlabDots + d];
-		plane_part[(size_t)(z - 1) * kSlabDots + d] = s;
-	}
+	double v[kSlabDots];
+	for (int d = 0; d < kSlabDots; d++) v[d] = chunk_part[((size_t)(z - 1) * kSlabChunks + lane) * kSlabDots + d];
+	warp_sum<kSlabDots>(v);
+	for (int d = 0; d < kSlabDots; d++)
+		if (lane == d) plane_part[(size_t)(z - 1) * kSlabDots + d] = v[d];
+}
+
+// The three dots of a sweep: plane rows summed in an order fixed by n3.
+__global__ void __launch_bounds__(kSlabThreads) k_slab_totals(long n3, const double *plane_part, double *out) {
+	double v[kSlabDots];
+	for (int d = 0; d < kSlabDots; d++) v[d] = 0.0;
+	for (long z = threadIdx.x; z < n3; z += blockDim.x)
+		for (int d = 0; d < kSlabDots; d++) v[d] += plane_part[z * kSlabDots + d];
+	block_total<kSlabDots>(v);
+	if (threadIdx.x == 0)
+		for (int d = 0; d < kSlabDots; d++) out[d] = v[d];
 }
 
 // t += x .* v, q += v .* v (stochastic-estimator.cc:195, :198); D = t ./ q (:216).
@@ -293,7 +313,7 @@ void launch_mode(SlabGeo g, Coef k, int z_lo, int z_hi, const sedi_slab_args &a,
 	for (int z = z_lo; z < z_hi; z += kMaxPlanes) {
 		const int ze = z_hi - z > kMaxPlanes ? z + kMaxPlanes : z_hi;
 		const dim3 grid(kSlabChunks, (unsigned)(ze - z));
-		k_slab_sweep<MODE><<<grid, kSlabThreads, 0, s>>>(g, k, z, ze, a, chunk);
+		k_slab_sweep<MODE><<<grid, block_threads(g.n1), 0, s>>>(g, k, z, ze, a, chunk);
 	}
 }
 
@@ -333,8 +353,19 @@ int sedi_slab_sweep(int mode, long n1, long n2, long nloc, double a, double b, d
 	case 11: launch_mode<11>(g, k, lo, hi, *args, chunk_part, s); break;
 	default: launch_mode<12>(g, k, lo, hi, *args, chunk_part, s); break;
 	}
-	if (dots) k_slab_plane_sums<<<(hi - lo + 127) / 128, 128, 0, s>>>(lo, hi, chunk_part, plane_part);
+	if (dots) k_slab_plane_sums<<<(hi - lo + 3) / 4, 128, 0, s>>>(lo, hi, chunk_part, plane_part);
 	return cudaGetLastError() == cudaSuccess ? 0 : SEDI_ERR_CUDA;
+}
+
+int sedi_slab_totals(long n3, const double *plane_part, double *scratch, double *totals, void *stream) {
+	if (n3 < 1 || !plane_part || !scratch || !totals) return SEDI_ERR_ARG;
+	cudaStream_t s = (cudaStream_t)stream;
+	k_slab_totals<<<1, kSlabThreads, 0, s>>>(n3, plane_part, scratch);
+	if (cudaGetLastError() != cudaSuccess ||
+	    cudaMemcpyAsync(totals, scratch, sizeof(double) * kSlabDots, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+	    cudaStreamSynchronize(s) != cudaSuccess)
+		return SEDI_ERR_CUDA;
+	return 0;
 }
 
 int sedi_slab_accumulate(long n, const double *x, const double *v, double *t, double *q, int reset, void *stream) {

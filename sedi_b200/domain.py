@@ -105,12 +105,15 @@ class GpuSlabBackend:
                                       ctypes.POINTER(_SlabArgs), vp, vp, vp]
         L.sedi_slab_accumulate.argtypes = [c_long, vp, vp, vp, vp, c_int, vp]
         L.sedi_slab_divide.argtypes = [c_long, vp, vp, vp, vp]
+        L.sedi_slab_totals.argtypes = [c_long, vp, vp, vp, vp]
         self.chunks = int(L.sedi_slab_chunks())
         self.n1, self.n2, self.n3 = (int(d) for d in dims)
         st = stencil or S.Stencil()
         self.coef = (st.a, st.b, st.c)
         self.device = device if device is not None else torch.device("cuda", torch.cuda.current_device())
         self._scratch = {}
+        self._tot = torch.empty(DOTS, dtype=torch.float64, device=self.device)
+        self._tot_host = torch.empty(DOTS, dtype=torch.float64, pin_memory=True)
 
     def _ptr(self, t):
         return ctypes.c_void_p(t.data_ptr()) if t is not None else None
@@ -144,9 +147,13 @@ class GpuSlabBackend:
         return self.torch.zeros((n3, DOTS), dtype=self.torch.float64, device=self.device)
 
     def totals(self, G):
-        """The three dot products: G summed over planes (device reduction of a
-        fixed shape, so of a fixed order), read back once."""
-        return tuple(G.sum(0).tolist())
+        """The three dot products: G summed over planes (one device reduction
+        in an order fixed by their number), read back once."""
+        rc = self.lib.sedi_slab_totals(G.shape[0], self._ptr(G), self._ptr(self._tot), self._ptr(self._tot_host),
+                                       self._stream())
+        if rc != 0:
+            raise RuntimeError(f"sedi_slab_totals failed ({rc})")
+        return tuple(self._tot_host.tolist())
 
     def sweep(self, mode, nloc, z_lo, z_hi, plane_part=None, first=False, **kw):
         """sedi_slab_sweep over ghosted planes [z_lo, z_hi): vectors (slab
