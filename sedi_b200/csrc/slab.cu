@@ -12,25 +12,31 @@
 // reference's zero ghost layer (Cg.hpp:57-62).
 //
 // Dot products are returned per plane, each summed in a fixed order that
-// depends only on n1 and n2 (the plane is cut into kSlabChunks row chunks,
-// one block each, then the chunks are added in order), so a plane's partial
+// depends only on n1 and n2 (the plane is cut into kSlabChunks row chunks, a
+// cluster of kSlabSplit blocks each, then the chunks are added in a fixed tree), so a plane's partial
 // sum is the same whichever rank holds the plane; the host adds the planes
 // in global order.  The solution therefore does not depend on the number of
 // slabs, bit for bit.  Elementwise values round as the reference's
 // (operator by operator, no FMA contraction), like the single-vector form:
 // a stencil input the reference stores (u = r .* iM, m = w .* iM, p_hat,
 // s_hat) is formed at each neighbour read with the same rounding.
+#include <cooperative_groups.h>
+
 #include "sedi_internal.h"
+
+namespace cg = cooperative_groups;
 
 namespace sedi {
 
 namespace {
 
 constexpr int kSlabThreads = 256;
-// Row chunks per plane, a block each (fixed: the summation order depends on
-// it).  A block's rows are a serial chain of loads: with 8 chunks a slab of
-// 192 x 160 x 64 gave 512 blocks of 20 rows, 43% of the warps an SM holds.
-constexpr int kSlabChunks = 32;
+constexpr int kSlabChunks = 8;  // row chunks per plane (fixed: the summation order depends on it)
+// Blocks (a cluster) of a chunk, which share its rows and add their sums through
+// distributed shared memory.  A block's rows are a serial chain of loads: one
+// block a chunk gave a slab of 192 x 160 x 64 512 blocks of 20 rows, 43% of the
+// warps an SM holds.
+constexpr int kSlabSplit = 4;
 constexpr int kSlabDots = 3;    // dot products per plane
 
 struct SlabGeo {
@@ -39,9 +45,10 @@ struct SlabGeo {
 };
 
 __device__ __forceinline__ void chunk_rows(const SlabGeo &g, int c, int *r0, int *r1) {
-	const int per = (g.n2 + kSlabChunks - 1) / kSlabChunks;
-	*r0 = c * per;
-	*r1 = min(g.n2, *r0 + per);
+	const int per = (g.n2 + kSlabChunks - 1) / kSlabChunks, sub = (per + kSlabSplit - 1) / kSlabSplit;
+	const int chunk = c / kSlabSplit, part = c % kSlabSplit, end = min(g.n2, (chunk + 1) * per);
+	*r0 = chunk * per + part * sub;
+	*r1 = min(end, *r0 + sub);
 }
 
 // 7-point stencil at ghosted plane z (1..nloc), row i2, column i1 of the
@@ -119,11 +126,10 @@ __host__ __device__ constexpr int mode_dots(int m) {
 }
 
 template <int MODE>
-__global__ void __launch_bounds__(kSlabThreads) k_slab_sweep(SlabGeo g, Coef k, int z_lo, int z_hi,
+__global__ void __cluster_dims__(kSlabSplit, 1, 1) __launch_bounds__(kSlabThreads) k_slab_sweep(SlabGeo g, Coef k, int z_lo, int z_hi,
                                                              sedi_slab_args a, double *chunk_part) {
-	const int z = z_lo + (int)blockIdx.y;
-	if (z >= z_hi) return;
-	const int c = blockIdx.x;
+	const int z = z_lo + (int)blockIdx.y;  // the grid has a row per plane
+	const int c = blockIdx.x;  // chunk * kSlabSplit + part
 	int r0, r1;
 	chunk_rows(g, c, &r0, &r1);
 	constexpr int ND = mode_dots(MODE) > 0 ? mode_dots(MODE) : 1;
@@ -229,23 +235,36 @@ __global__ void __launch_bounds__(kSlabThreads) k_slab_sweep(SlabGeo g, Coef k, 
 	}
 	if (mode_dots(MODE) == 0) return;
 	block_total<ND>(v);
-	if (threadIdx.x == 0) {
-		double *o = chunk_part + ((size_t)(z - 1) * kSlabChunks + c) * kSlabDots;
+	// The chunk's blocks hand their sums to the first of them, which adds them in order.
+	__shared__ double part[kSlabSplit][ND];
+	cg::cluster_group cluster = cg::this_cluster();
+	if (threadIdx.x == 0)
+#pragma unroll
+		for (int d = 0; d < ND; d++) cluster.map_shared_rank(&part[c % kSlabSplit][d], 0)[0] = v[d];
+	cluster.sync();
+	if (c % kSlabSplit == 0 && threadIdx.x == 0) {
+#pragma unroll
+		for (int d = 0; d < ND; d++) {
+			v[d] = 0.0;
+			for (int k = 0; k < kSlabSplit; k++) v[d] += part[k][d];
+		}
+		double *o = chunk_part + ((size_t)(z - 1) * kSlabChunks + c / kSlabSplit) * kSlabDots;
 		for (int d = 0; d < kSlabDots; d++) o[d] = d < mode_dots(MODE) ? v[d < ND ? d : 0] : 0.0;
 	}
 }
 
-// Per-plane sums of the chunk partials in a fixed tree: a warp per plane, a
-// lane per chunk.
+// Per-plane sums of the chunk partials in a fixed tree: a lane per chunk, four
+// planes a warp.
 __global__ void __launch_bounds__(128) k_slab_plane_sums(int z_lo, int z_hi, const double *chunk_part, double *plane_part) {
-	static_assert(kSlabChunks == 32, "a lane per chunk");
-	const int z = z_lo + (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
-	if (z >= z_hi) return;
+	static_assert(kSlabChunks == 8, "eight lanes a plane");
+	const int z = z_lo + (int)((blockIdx.x * blockDim.x + threadIdx.x) / kSlabChunks), c = threadIdx.x % kSlabChunks;
 	double v[kSlabDots];
-	for (int d = 0; d < kSlabDots; d++) v[d] = chunk_part[((size_t)(z - 1) * kSlabChunks + lane) * kSlabDots + d];
-	warp_sum<kSlabDots>(v);
 	for (int d = 0; d < kSlabDots; d++)
-		if (lane == d) plane_part[(size_t)(z - 1) * kSlabDots + d] = v[d];
+		v[d] = z < z_hi ? chunk_part[((size_t)(z - 1) * kSlabChunks + c) * kSlabDots + d] : 0.0;
+	for (int off = kSlabChunks / 2; off > 0; off >>= 1)
+		for (int d = 0; d < kSlabDots; d++) v[d] += __shfl_xor_sync(0xffffffffu, v[d], off);
+	for (int d = 0; d < kSlabDots; d++)
+		if (z < z_hi && c == d) plane_part[(size_t)(z - 1) * kSlabDots + d] = v[d];
 }
 
 // The three dots of a sweep: plane rows summed in an order fixed by n3.
@@ -312,7 +331,7 @@ void launch_mode(SlabGeo g, Coef k, int z_lo, int z_hi, const sedi_slab_args &a,
 	constexpr int kMaxPlanes = 65535;  // grid y limit: one block row per plane
 	for (int z = z_lo; z < z_hi; z += kMaxPlanes) {
 		const int ze = z_hi - z > kMaxPlanes ? z + kMaxPlanes : z_hi;
-		const dim3 grid(kSlabChunks, (unsigned)(ze - z));
+		const dim3 grid(kSlabChunks * kSlabSplit, (unsigned)(ze - z));
 		k_slab_sweep<MODE><<<grid, block_threads(g.n1), 0, s>>>(g, k, z, ze, a, chunk);
 	}
 }
@@ -353,7 +372,7 @@ int sedi_slab_sweep(int mode, long n1, long n2, long nloc, double a, double b, d
 	case 11: launch_mode<11>(g, k, lo, hi, *args, chunk_part, s); break;
 	default: launch_mode<12>(g, k, lo, hi, *args, chunk_part, s); break;
 	}
-	if (dots) k_slab_plane_sums<<<(hi - lo + 3) / 4, 128, 0, s>>>(lo, hi, chunk_part, plane_part);
+	if (dots) k_slab_plane_sums<<<(hi - lo + 15) / 16, 128, 0, s>>>(lo, hi, chunk_part, plane_part);
 	return cudaGetLastError() == cudaSuccess ? 0 : SEDI_ERR_CUDA;
 }
 
