@@ -144,6 +144,44 @@ __device__ __forceinline__ float st7r(float a, float b, float c, float xc, float
 	return y;
 }
 
+// Where a block's ghost rows are: {shared offset of the row's first point, its
+// place in the neighbour's faces relative to the block's own}, built once, so
+// that an iteration spends no index arithmetic on them (dealt out and decoded
+// in place they cost 50 instructions a row and thread, a fifth of all).
+// `nbr`: neighbours, bit 0 i2 low, 1 i2 high, 2 i3 low, 3 i3 high.
+__device__ __forceinline__ void ghost_table(const ResArgs &A, int2 *tab, int *count, int B2, int nd, int nr, unsigned nbr,
+                                            int pitch, int pp, int face_rows) {
+	const int t = threadIdx.x, n1 = A.n1;
+	int n = 0;
+	if (nbr & 1u) {  // row -1, from the high i2 face of the block below
+		for (int j = t; j < nd; j += blockDim.x) tab[n + j] = make_int2((j + 1) * pp + 1, (A.nd + j - face_rows) * n1);
+		n += nd;
+	}
+	if (nbr & 2u) {
+		for (int j = t; j < nd; j += blockDim.x)
+			tab[n + j] = make_int2((j + 1) * pp + (nr + 1) * pitch + 1, (face_rows + j) * n1);
+		n += nd;
+	}
+	if (nbr & 4u) {  // plane -1, from the high i3 face
+		for (int j = t; j < nr; j += blockDim.x)
+			tab[n + j] = make_int2((j + 1) * pitch + 1, (2 * A.nd + B2 + j - A.s2 * face_rows) * n1);
+		n += nr;
+	}
+	if (nbr & 8u) {
+		for (int j = t; j < nr; j += blockDim.x)
+			tab[n + j] = make_int2((nd + 1) * pp + (j + 1) * pitch + 1, (2 * A.nd + j + A.s2 * face_rows) * n1);
+		n += nr;
+	}
+	if (t == 0) *count = n;
+}
+// Bytes of shared memory before the table: `ghosted` fields with ghosts and
+// `own` fields of the block's own points.
+__host__ __device__ __forceinline__ size_t ghost_table_offset(const ResArgs &A, size_t elem, int ghosted, int own, int B2, int T) {
+	const size_t e = (size_t)(A.n1 + 1) * (B2 + 2) * (A.nd + 2) + 1;
+	return ((e * ghosted + (size_t)own * A.nd * T) * elem + 7) / 8 * 8;
+}
+__host__ __device__ __forceinline__ size_t ghost_table_bytes(int B2, int nd) { return 8 + 8 * (size_t)(2 * nd + 2 * B2); }
+
 // Uniform state of the solve a block runs, in shared memory: written by warp 0
 // at the end of a group sum, read by every thread after it.  Registers are
 // left to the Krylov fields.
@@ -191,7 +229,8 @@ __global__ void __launch_bounds__(TMAX, BLOCKS) k_res_cg(const __grid_constant__
 	V *const sp = reinterpret_cast<V *>(smem);
 	const int group = blockIdx.x / A.G;
 	const int s3 = n1 * A.n2;  // the grid has far fewer than 2^31 points
-	int nd, rows, so, go, own3, lo_c, hi_c, lo_d, hi_d;
+	int nd, rows, so, go, own3, hi_c, hi_d;
+	bool lo_c, lo_d;
 	unsigned nbr;  // neighbours: bit 0 i2 low, 1 i2 high, 2 i3 low, 3 i3 high; box rows above
 	{
 		const int m = blockIdx.x % A.G;
@@ -203,9 +242,9 @@ __global__ void __launch_bounds__(TMAX, BLOCKS) k_res_cg(const __grid_constant__
 		own3 = (2 * A.nd + rg * C) * n1 + i1;                 // and in the low i3 face
 		const bool lo2 = row0 > 0, hi2 = row0 + nr < A.n2, lo3 = z0 > 0, hi3 = z0 + nd < A.n3;
 		nbr = (lo2 ? 1u : 0u) | (hi2 ? 2u : 0u) | (lo3 ? 4u : 0u) | (hi3 ? 8u : 0u) | (unsigned)nr << 4;
-		lo_c = lo2 && rg == 0 ? 0 : -1;  // published rows and planes
+		lo_c = lo2 && rg == 0;  // published rows and planes: the first, and which of the last
 		hi_c = hi2 ? nr - 1 - rg * C : -1;
-		lo_d = lo3 ? 0 : -1;
+		lo_d = lo3;
 		hi_d = hi3 ? nd - 1 : -1;
 		if (t == 0) {
 			g->G = A.G;
@@ -219,6 +258,9 @@ __global__ void __launch_bounds__(TMAX, BLOCKS) k_res_cg(const __grid_constant__
 	const int face_rows = 2 * A.nd + 2 * B2;  // face rows of a block: i2 low, high, i3 low, high
 	unsigned round = 0;                       // group sums so far
 	V *const faces = static_cast<V *>(A.edge) + (size_t)blockIdx.x * face_rows * n1;  // this block's
+	int *const ghost_count = reinterpret_cast<int *>(smem + ghost_table_offset(A, sizeof(V), 1, 0, B2, blockDim.x));
+	int2 *const ghost_rows = reinterpret_cast<int2 *>(ghost_count + 2);
+	ghost_table(A, ghost_rows, ghost_count, B2, nd, (int)(nbr >> 4), nbr, pitch, pp, face_rows);
 	const S im = (S)A.iM;
 
 	const int units = (A.lanes + NL - 1) / NL;
@@ -280,9 +322,9 @@ __global__ void __launch_bounds__(TMAX, BLOCKS) k_res_cg(const __grid_constant__
 		// Publishes a point of the box's faces (f2, f3: the thread's place in the
 		// i2 and i3 faces) for the neighbours to read after the next fenced sum.
 		auto publish = [&](int c, int d, int f2, int f3, const V &v) {
-			if (c == lo_c) stl2(faces + f2, v);
+			if (c == 0 && lo_c) stl2(faces + f2, v);
 			if (c == hi_c) stl2(faces + f2 + A.nd * n1, v);
-			if (d == lo_d) stl2(faces + f3 + c * n1, v);
+			if (d == 0 && lo_d) stl2(faces + f3 + c * n1, v);
 			if (d == hi_d) stl2(faces + f3 + (B2 + c) * n1, v);
 		};
 		auto publish_all = [&]() {
@@ -348,37 +390,18 @@ __global__ void __launch_bounds__(TMAX, BLOCKS) k_res_cg(const __grid_constant__
 				S be[NL];
 #pragma unroll
 				for (int l = 0; l < NL; l++) be[l] = (S)st.beta[l];
-				// Ghost rows: nd on each i2 side, nr on each i3 side, dealt to the row groups.
-				const int nr = (int)(nbr >> 4), ghosts = 2 * nd + 2 * nr;
+				const int ghosts = *ghost_count;
 				constexpr int HB = 6;
-				for (int h0 = rg; h0 < ghosts; h0 += HB * A.RG) {
+				for (int h0 = rg; h0 < ghosts; h0 += HB * A.RG) {  // dealt to the row groups
 					V rh[HB];
 					int off[HB];
 #pragma unroll
 					for (int k = 0; k < HB; k++) {
-						const int h = h0 + k * A.RG;
 						off[k] = -1;
-						if (h >= ghosts) continue;
-						// Ghost row h: box row j2 and plane j3 (-1 and nr / nd outside the
-						// box), the face row of the neighbour it comes from.
-						int j2, j3, fr;
-						unsigned side;
-						if (h < 2 * nd) {
-							const bool hi = h >= nd;
-							j3 = hi ? h - nd : h;
-							j2 = hi ? nr : -1;
-							side = hi ? 2u : 1u;
-							fr = hi ? face_rows + j3 : -face_rows + A.nd + j3;
-						} else {
-							const bool hi = h >= 2 * nd + nr;
-							j2 = hi ? h - 2 * nd - nr : h - 2 * nd;
-							j3 = hi ? nd : -1;
-							side = hi ? 8u : 4u;
-							fr = 2 * A.nd + j2 + (hi ? A.s2 * face_rows : B2 - A.s2 * face_rows);
-						}
-						if (!(nbr & side)) continue;
-						off[k] = (j3 + 1) * pp + (j2 + 1) * pitch + 1 + i1;
-						rh[k] = ldl2(faces + fr * n1 + i1);
+						if (h0 + k * A.RG >= ghosts) continue;
+						const int2 e = ghost_rows[h0 + k * A.RG];
+						off[k] = e.x + i1;
+						rh[k] = ldl2(faces + e.y + i1);
 					}
 #pragma unroll
 					for (int k = 0; k < HB; k++) {
@@ -727,39 +750,26 @@ struct ResBox {
 	// Ghost points of the box, HB rows of a thread at a time: load(k, from) of
 	// the neighbour's face point, then use(k, shared offset).
 	template <int HB, class Load, class Use>
-	__device__ __forceinline__ void ghosts(const ResArgs &A, Load load, Use use) const {
+	__device__ __forceinline__ void ghosts(const ResArgs &A, const int2 *tab, int count, Load load, Use use) const {
 		if (rg >= A.RG) return;
-		const int n = 2 * nd + 2 * nr;
-		for (int h0 = rg; h0 < n; h0 += HB * A.RG) {
+		for (int h0 = rg; h0 < count; h0 += HB * A.RG) {
 			int off[HB];
 #pragma unroll
 			for (int k = 0; k < HB; k++) {
-				const int h = h0 + k * A.RG;
 				off[k] = -1;
-				if (h >= n) continue;
-				int j2, j3, fr;  // box row and plane (-1, nr / nd outside), face row of the neighbour
-				bool there;
-				if (h < 2 * nd) {
-					const bool hi = h >= nd;
-					j3 = hi ? h - nd : h;
-					j2 = hi ? nr : -1;
-					there = hi ? hi2 : lo2;
-					fr = hi ? face_rows + j3 : A.nd + j3 - face_rows;
-				} else {
-					const bool hi = h >= 2 * nd + nr;
-					j2 = hi ? h - 2 * nd - nr : h - 2 * nd;
-					j3 = hi ? nd : -1;
-					there = hi ? hi3 : lo3;
-					fr = 2 * A.nd + j2 + (hi ? A.s2 * face_rows : A.RG - A.s2 * face_rows);
-				}
-				if (!there) continue;
-				off[k] = (j3 + 1) * pp + (j2 + 1) * pitch + 1 + i1;
-				load(k, fr * A.n1 + i1);
+				if (h0 + k * A.RG >= count) continue;
+				const int2 e = tab[h0 + k * A.RG];
+				off[k] = e.x + i1;
+				load(k, e.y + i1);
 			}
 #pragma unroll
 			for (int k = 0; k < HB; k++)
 				if (off[k] >= 0) use(k, off[k]);
 		}
+	}
+	__device__ void table(const ResArgs &A, int2 *tab, int *count) const {
+		ghost_table(A, tab, count, A.RG, nd, nr, (lo2 ? 1u : 0u) | (hi2 ? 2u : 0u) | (lo3 ? 4u : 0u) | (hi3 ? 8u : 0u), pitch, pp,
+		            face_rows);
 	}
 	// f(d, centre, A (scale .* field)) of the thread's points; SCALED as the
 	// reference stores the stencil input (each value read times scale).
@@ -880,6 +890,9 @@ __global__ void __launch_bounds__(TMAX, 1) k_res_pcg(const __grid_constant__ Res
 	double *const faces = static_cast<double *>(A.edge) + (size_t)blockIdx.x * B.face_rows * A.n1;
 	const size_t other = (size_t)gridDim.x * B.face_rows * A.n1;
 	if (t == 0) group_init(g, A);
+	int *const ghost_count = reinterpret_cast<int *>(smem + ghost_table_offset(A, sizeof(double), 1, A.nsm, A.RG, T));
+	int2 *const ghost_rows = reinterpret_cast<int2 *>(ghost_count + 2);
+	B.table(A, ghost_rows, ghost_count);
 	unsigned round = 0;
 	const double im = A.iM;
 	for (int unit = blockIdx.x / A.G; unit < A.lanes; unit += A.groups) {
@@ -939,7 +952,7 @@ __global__ void __launch_bounds__(TMAX, 1) k_res_pcg(const __grid_constant__ Res
 			}
 		};
 		if (!st.done) {
-			B.ghosts<HB>(A, load, put);
+			B.ghosts<HB>(A, ghost_rows, *ghost_count, load, put);
 			__syncthreads();
 			double v[3] = {0.0, 0.0, 0.0};
 			B.march<D, UNIT, false>(A, sm, 1.0, [&](int d, double, double wi) {  // w = A u (:141-143)
@@ -962,7 +975,7 @@ __global__ void __launch_bounds__(TMAX, 1) k_res_pcg(const __grid_constant__ Res
 			for (int it = 1; !st.done; it++) {
 				in = faces + (it & 1) * other;
 				out = faces + (~it & 1) * other;
-				B.ghosts<HB>(A, load, put);
+				B.ghosts<HB>(A, ghost_rows, *ghost_count, load, put);
 				__syncthreads();
 				const double alpha = st.alpha, beta = st.beta;
 				v[0] = v[1] = v[2] = 0.0;
@@ -1032,6 +1045,9 @@ __global__ void __launch_bounds__(TMAX, 1) k_res_bicg(const __grid_constant__ Re
 	const size_t other = (size_t)gridDim.x * B.face_rows * A.n1;
 	const double *vin = nullptr;
 	if (t == 0) group_init(g, A);
+	int *const ghost_count = reinterpret_cast<int *>(smem + ghost_table_offset(A, sizeof(double), 2, A.nsm, A.RG, T));
+	int2 *const ghost_rows = reinterpret_cast<int2 *>(ghost_count + 2);
+	B.table(A, ghost_rows, ghost_count);
 	unsigned round = 0;
 	const double im = A.iM;
 	constexpr int HB = 4;
@@ -1078,8 +1094,8 @@ __global__ void __launch_bounds__(TMAX, 1) k_res_bicg(const __grid_constant__ Re
 				auto new_p = [&](double ri, double pi, double vi) {
 					return first ? ri : add(add(ri, mul(beta, pi)), mul(bo, vi));  // :168, :171
 				};
-				if (first) B.ghosts<HB>(A, load_r, [&](int k, int off) { sp[off] = hr[k]; });
-				else B.ghosts<HB>(A, load_rv, [&](int k, int off) { sp[off] = new_p(hr[k], sp[off], hw[k]); });
+				if (first) B.ghosts<HB>(A, ghost_rows, *ghost_count, load_r, [&](int k, int off) { sp[off] = hr[k]; });
+				else B.ghosts<HB>(A, ghost_rows, *ghost_count, load_rv, [&](int k, int off) { sp[off] = new_p(hr[k], sp[off], hw[k]); });
 				if (B.own)
 #pragma unroll
 					for (int d = 0; d < D; d++)
@@ -1103,7 +1119,7 @@ __global__ void __launch_bounds__(TMAX, 1) k_res_bicg(const __grid_constant__ Re
 			const double alpha = st.alpha;
 			vin = vnew;
 			{
-				B.ghosts<HB>(A, load_rv, [&](int k, int off) { ss[off] = add(hr[k], mul(-alpha, hw[k])); });  // :189
+				B.ghosts<HB>(A, ghost_rows, *ghost_count, load_rv, [&](int k, int off) { ss[off] = add(hr[k], mul(-alpha, hw[k])); });  // :189
 				if (B.own)
 #pragma unroll
 					for (int d = 0; d < D; d++)
@@ -1252,7 +1268,8 @@ Plan plan_for(int ks, const Geo &g, int units, int sms, size_t smem_max, double 
 			const int T = (RG * g.n1 + 31) / 32 * 32, B2 = RG * C, s2 = (g.n2 + B2 - 1) / B2;
 			for (int nd = 1; nd <= kShapeD[sh] && nd <= g.n3; nd++) {
 				const long long G = (long long)s2 * ((g.n3 + nd - 1) / nd);
-				const size_t ghosted = ((size_t)(g.n1 + 1) * (B2 + 2) * (nd + 2) + 1) * kGhosted[ks] * 8, own = (size_t)nd * T * 8;
+				const size_t ghosted = ((size_t)(g.n1 + 1) * (B2 + 2) * (nd + 2) + 1) * kGhosted[ks] * 8 + ghost_table_bytes(B2, nd),
+				             own = (size_t)nd * T * 8;
 				int nsm = kOwn[ks];
 				if (sh == kShapes - 1)
 					while (nsm > (ks == SEDI_BICGSTAB ? 1 : 0) && ghosted + nsm * own > smem_max) nsm--;
