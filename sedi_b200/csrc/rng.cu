@@ -66,46 +66,50 @@ __device__ __forceinline__ uint32_t mt_temper(uint32_t y) {
 	return y;
 }
 
-// Twist phase over words [lo, hi): every thread first reads its inputs, then
-// all write.
-__device__ __forceinline__ void mt_phase(uint32_t *mt, int lo, int hi) {
-	uint32_t v[(kMtN + kMtThreads - 1) / kMtThreads];
-	int k = 0;
-	for (int i = lo + threadIdx.x; i < hi; i += kMtThreads, k++)
-		v[k] = mt_mix(mt[i], mt[(i + 1) % kMtN], mt[(i + kMtM) % kMtN]);
-	__syncthreads();
-	k = 0;
-	for (int i = lo + threadIdx.x; i < hi; i += kMtThreads, k++) mt[i] = v[k];
-	__syncthreads();
-}
-
 // Probe j (seed0 + j) of a batch, written as lane j of a lane-sliced FP64
 // field (element (i, j) at ((j / W) * npts + i) * W + j % W), or densely at
-// out[j * npts + i] when W == 0.
+// out[j * npts + i] when W == 0.  A probe is a serial chain of twists of 312
+// points each, bound by its barriers: the new state goes to a second buffer,
+// so a phase needs one barrier (its inputs are the old state and the phase
+// before), and a word is tempered where it is made: four barriers a twist
+// instead of eight.
 __global__ void __launch_bounds__(kMtThreads) k_mt_probes(uint32_t seed0, long long npts, int W, double *out) {
-	__shared__ uint32_t mt[kMtN];
+	__shared__ uint32_t state[2][kMtN];
 	__shared__ uint32_t draw[kMtN];
-	const int j = blockIdx.x;
-	if (threadIdx.x == 0) {
-		mt[0] = seed0 + (uint32_t)j;
-		for (int i = 1; i < kMtN; i++) mt[i] = 1812433253u * (mt[i - 1] ^ (mt[i - 1] >> 30)) + (uint32_t)i;
+	const int j = blockIdx.x, t = threadIdx.x;
+	if (t == 0) {
+		uint32_t x = seed0 + (uint32_t)j;
+		state[0][0] = x;
+		for (int i = 1; i < kMtN; i++) state[0][i] = x = 1812433253u * (x ^ (x >> 30)) + (uint32_t)i;
 	}
 	__syncthreads();
 	double *base = W ? out + ((long long)(j / W) * npts) * W + (j % W) : out + (long long)j * npts;
 	const long long step = W ? W : 1;
+	constexpr int kPhase = kMtN - kMtM;  // 227 words a phase, by a thread each
+	static_assert(kPhase <= kMtThreads && 3 * kPhase >= kMtN, "phases");
+	uint32_t *old = state[0], *now = state[1];
 	for (long long p0 = 0; p0 < npts; p0 += kMtN / 2) {
-		mt_phase(mt, 0, kMtN - kMtM);
-		mt_phase(mt, kMtN - kMtM, 2 * (kMtN - kMtM));
-		mt_phase(mt, 2 * (kMtN - kMtM), kMtN);
-		for (int i = threadIdx.x; i < kMtN; i += kMtThreads) draw[i] = mt_temper(mt[i]);
-		__syncthreads();
-		for (int k = threadIdx.x; k < kMtN / 2; k += kMtThreads) {
+#pragma unroll
+		for (int ph = 0; ph < 3; ph++) {
+			const int i = ph * kPhase + t;
+			if (t < kPhase && i < kMtN) {
+				const uint32_t next = i + 1 < kMtN ? old[i + 1] : now[0];
+				const uint32_t w = mt_mix(old[i], next, ph == 0 ? old[i + kMtM] : now[i - kPhase]);
+				now[i] = w;
+				draw[i] = mt_temper(w);
+			}
+			__syncthreads();
+		}
+		for (int k = t; k < kMtN / 2; k += kMtThreads) {
 			const long long p = p0 + k;
 			if (p >= npts) break;
 			const double sum = __dadd_rn((double)draw[2 * k], __dmul_rn((double)draw[2 * k + 1], 4294967296.0));
 			base[p * step] = sum > 9223372036854775808.0 ? 1.0 : -1.0;
 		}
-		__syncthreads();
+		uint32_t *const s = old;
+		old = now;
+		now = s;
+		__syncthreads();  // draw is rewritten by the next twist
 	}
 }
 
