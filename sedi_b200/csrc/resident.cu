@@ -1321,10 +1321,13 @@ size_t edge_bytes(int ks, const Plan &p, const Geo &g) {
 
 struct Resident {
 	Plan plan;
+	int units = 0;          // solves the plan is for
 	int ks = 0;
 	bool fp32 = false, unit = false;
-	Word2 *words = nullptr;
-	void *edge = nullptr;
+	size_t shared = 0;      // shared memory of a block, at most
+	bool ready[kShapes] = {};
+	void *buf = nullptr;    // the groups' reduction words, then the boxes' faces
+	size_t buf_bytes = 0;
 	unsigned long long launch = 0;
 	int device = 0, sms = 0;
 	cudaEvent_t done = nullptr;  // after the latest launch
@@ -1346,6 +1349,50 @@ static void running_remove(Resident *R) {
 			g_running.erase(g_running.begin() + (long)i);
 			return;
 		}
+}
+
+// Plan for `units` solves, chosen by their number and the grid alone (so a
+// result does not depend on the context's room for more): 10 FP64 solves of
+// 58^3 on a plan for 16 ran as 9 groups and one more round.  The one in use
+// stays where the kernel of a better one cannot run.
+static int use_plan(Ctx *c, Resident *R, int units) {
+	if (units == R->units) return 0;
+	double cycles = 0.0;
+	const Plan p = plan_for(R->ks, c->g, units, R->sms, R->shared, &cycles);
+	if (p.shape < 0) return 0;
+	if (!R->ready[p.shape]) {
+		const void *const k = (const void *)kernel_for(R->ks, R->fp32, R->unit, p.shape);
+		int per_sm = 0;
+		// (The attribute is the kernel's, whoever launches it: its largest use.)
+		if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(R->shared / kShapeB[p.shape])) !=
+		        cudaSuccess ||
+		    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kShapeT[p.shape], R->shared / kShapeB[p.shape]) !=
+		        cudaSuccess ||
+		    per_sm < kShapeB[p.shape]) {
+			cudaGetLastError();
+			return 0;
+		}
+		R->ready[p.shape] = true;
+	}
+	const size_t bytes = word_bytes(p) + edge_bytes(R->ks, p, c->g);
+	if (bytes > R->buf_bytes) {
+		if (R->buf) cudaFree(R->buf);
+		R->buf = nullptr;
+		R->buf_bytes = 0;
+		R->units = 0;
+		if (cudaMalloc(&R->buf, bytes) != cudaSuccess) {
+			cudaGetLastError();
+			c->error = "device allocation failed (resident solver)";
+			return SEDI_ERR_NOMEM;
+		}
+		R->buf_bytes = bytes;
+		// No word may carry a stamp of a launch to come.
+		const cudaError_t e = cudaMemsetAsync(R->buf, 0, bytes, c->stream);
+		if (e != cudaSuccess) return set_cuda_error(c, e, "resident solver");
+	}
+	R->plan = p;
+	R->units = units;
+	return 0;
 }
 
 // A resident solver for `lanes` right-hand sides of the context's grid; *out
@@ -1375,33 +1422,20 @@ int resident_alloc(Ctx *c, int ks, bool fp32, int lanes, Resident **out) {
 	// and 20), a batch does.
 	if (fp32) cycles *= 1.8;
 	if (lanes > 1 && cycles > stream_cycles(ks, c->g, lanes, fp32)) return 0;
-	const ResKernel k = kernel_for(ks, fp32, unit, p.shape);
-	int per_sm = 0;
-	// (The attribute is the kernel's, whoever launches it: its largest use.)
-	if (cudaFuncSetAttribute((const void *)k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-	                         (int)(shared / kShapeB[p.shape])) != cudaSuccess ||
-	    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void *)k, p.T, p.smem) != cudaSuccess || per_sm < kShapeB[p.shape]) {
-		cudaGetLastError();
-		return 0;
-	}
 	Resident *R = new (std::nothrow) Resident();
 	if (!R) return SEDI_ERR_NOMEM;
-	R->plan = p;
 	R->ks = ks;
 	R->fp32 = fp32;
 	R->unit = unit;
+	R->shared = shared;
 	R->device = c->device;
 	R->sms = sms;
-	if (cudaMalloc(&R->words, word_bytes(p)) != cudaSuccess || cudaMalloc(&R->edge, edge_bytes(ks, p, c->g)) != cudaSuccess ||
-	    cudaEventCreateWithFlags(&R->done, cudaEventDisableTiming) != cudaSuccess) {
+	const int rc = use_plan(c, R, fp32 ? (lanes + 1) / 2 : lanes);
+	if (rc || R->plan.shape < 0 || cudaEventCreateWithFlags(&R->done, cudaEventDisableTiming) != cudaSuccess) {
 		cudaGetLastError();
 		resident_free(R);
-		c->error = "device allocation failed (resident solver)";
-		return SEDI_ERR_NOMEM;
+		return rc;
 	}
-	// No word may carry a stamp of a launch to come.
-	cudaMemsetAsync(R->words, 0, word_bytes(p), c->stream);
-	cudaMemsetAsync(R->edge, 0, edge_bytes(ks, p, c->g), c->stream);
 	*out = R;
 	return cudaStreamSynchronize(c->stream) == cudaSuccess ? 0 : set_cuda_error(c, cudaGetLastError(), "resident_alloc");
 }
@@ -1413,16 +1447,18 @@ void resident_free(Resident *R) {
 		running_remove(R);
 	}
 	if (R->done) cudaEventDestroy(R->done);
-	if (R->words) cudaFree(R->words);
-	if (R->edge) cudaFree(R->edge);
+	if (R->buf) cudaFree(R->buf);
 	delete R;
 }
 
 // Solves io.lanes right-hand sides on the context's stream.
 int resident_launch(Ctx *c, Resident *R, const ResIO &io) {
-	const Plan &p = R->plan;
-	const int units = R->fp32 ? (io.lanes + 1) / 2 : io.lanes, groups = units < p.groups ? units : p.groups;
+	const int units = R->fp32 ? (io.lanes + 1) / 2 : io.lanes;
 	if (units < 1) return 0;
+	const int rc = use_plan(c, R, units);
+	if (rc) return rc;
+	const Plan &p = R->plan;
+	const int groups = units < p.groups ? units : p.groups;
 	ResArgs a;
 	a.n1 = c->g.n1;
 	a.n2 = c->g.n2;
@@ -1443,8 +1479,8 @@ int resident_launch(Ctx *c, Resident *R, const ResIO &io) {
 	a.rhs = io.rhs;
 	a.x = io.x;
 	a.xlo = (float2 *)io.xlo;
-	a.edge = R->edge;
-	a.words = R->words;
+	a.words = (Word2 *)R->buf;
+	a.edge = (char *)R->buf + word_bytes(p);
 	a.stamp = ++R->launch << 36;
 	a.tol = io.tol;
 	a.tol_in = io.tol_in;
