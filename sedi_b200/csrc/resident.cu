@@ -41,7 +41,7 @@ struct ResArgs {
 	const double *rhs;    // right-hand sides
 	double *x;            // FP64: x (in: first guess); FP32: x_hi
 	float2 *xlo;          // FP32: correction since the last reliable update
-	void *edge;           // boundary rows: [fields][groups][G][2 nd + 2 RG*C][n1] of V
+	void *edge;           // boundary rows: [fields][groups][G][2 nd + 2 RG*C][n1] of Face
 	Word2 *words;         // [groups][res_words(G)]: the groups' reductions
 	unsigned long long stamp;  // stamps of this launch lie above it
 	double *scratch[4];   // own-point fields that do not fit shared memory: q, s, p, z (pipelined CG)
@@ -86,6 +86,48 @@ template <>
 __device__ __forceinline__ float2 lane_zero<float2>() {
 	return make_float2(0.f, 0.f);
 }
+
+__device__ __forceinline__ unsigned long long bits(double v) { return __double_as_longlong(v); }
+__device__ __forceinline__ unsigned long long bits(const float2 &v) {
+	return (unsigned long long)__float_as_uint(v.y) << 32 | __float_as_uint(v.x);
+}
+template <class V>
+__device__ __forceinline__ V value(unsigned long long b);
+template <>
+__device__ __forceinline__ double value<double>(unsigned long long b) {
+	return __longlong_as_double(b);
+}
+template <>
+__device__ __forceinline__ float2 value<float2>(unsigned long long b) {
+	return make_float2(__uint_as_float((unsigned)b), __uint_as_float((unsigned)(b >> 32)));
+}
+
+// A point of a block's faces.  Plain (S false): written through L1 and made
+// visible by a fenced group sum.  Stamped (S true): value and stamp of its
+// publication in one atomic exchange, so the sum needs no fence (800-900 cycles
+// for the stores, 300 for the reader) and a reader that comes too early waits
+// for the stamp.  Exchanges are slower per point, so boxes with few planes
+// take them.
+template <class V, bool S>
+struct Face;
+template <class V>
+struct Face<V, false> {
+	V v;
+	__device__ __forceinline__ void put(const V &x, unsigned long long) { stl2(&v, x); }
+	typedef V Got;
+	__device__ __forceinline__ Got load() const { return ldl2(&v); }
+	__device__ __forceinline__ V get(const Got &g, unsigned long long, ResGroup *) const { return g; }
+};
+template <class V>
+struct Face<V, true> {
+	Word2 w;
+	__device__ __forceinline__ void put(const V &x, unsigned long long stamp) { swap2(&w, bits(x), stamp); }
+	typedef Word2 Got;
+	__device__ __forceinline__ Got load() const { return load2(&w); }
+	__device__ __forceinline__ V get(const Got &g, unsigned long long stamp, ResGroup *gr) const {
+		return value<V>(g.b == stamp ? g.a : wait2(&w, stamp, gr).a);
+	}
+};
 
 // r iM + beta p, and x + a y: FP64 rounds each operator, FP32 fuses.
 __device__ __forceinline__ double comb(double r, double im, double beta, double p) {
@@ -182,6 +224,11 @@ __host__ __device__ __forceinline__ size_t ghost_table_offset(const ResArgs &A, 
 }
 __host__ __device__ __forceinline__ size_t ghost_table_bytes(int B2, int nd) { return 8 + 8 * (size_t)(2 * nd + 2 * B2); }
 
+// CG's boxes of one row a thread have stamped faces (32^3: 5.6 -> 5.4 us an
+// iteration, 48^3 6.2 -> 5.9); larger ones publish too many points, and
+// pipelined CG and BiCGStab gained nothing (64^3: 5.1 -> 5.4, 11.2 -> 12.2 us).
+__host__ __device__ constexpr bool stamped(int ks, int C) { return ks == SEDI_CG && C == 1; }
+
 // Uniform state of the solve a block runs, in shared memory: written by warp 0
 // at the end of a group sum, read by every thread after it.  Registers are
 // left to the Krylov fields.
@@ -219,6 +266,8 @@ __global__ void __launch_bounds__(TMAX, BLOCKS) k_res_cg(const __grid_constant__
 	constexpr int NL = Lanes<V>::N;
 	constexpr bool MIXED = NL == 2;
 	constexpr bool KEEP = C * D <= 16;  // A p stays in registers between its two uses
+	constexpr bool STAMP = stamped(SEDI_CG, C);
+	typedef Face<V, STAMP> FaceT;
 	extern __shared__ __align__(16) unsigned char smem[];
 	__shared__ ResGroup gsh;
 	__shared__ CgState<NL> st;
@@ -257,7 +306,8 @@ __global__ void __launch_bounds__(TMAX, BLOCKS) k_res_cg(const __grid_constant__
 	}
 	const int face_rows = 2 * A.nd + 2 * B2;  // face rows of a block: i2 low, high, i3 low, high
 	unsigned round = 0;                       // group sums so far
-	V *const faces = static_cast<V *>(A.edge) + (size_t)blockIdx.x * face_rows * n1;  // this block's
+	unsigned pub = 0;                         // publications of face rows
+	FaceT *const faces = static_cast<FaceT *>(A.edge) + (size_t)blockIdx.x * face_rows * n1;  // this block's
 	int *const ghost_count = reinterpret_cast<int *>(smem + ghost_table_offset(A, sizeof(V), 1, 0, B2, blockDim.x));
 	int2 *const ghost_rows = reinterpret_cast<int2 *>(ghost_count + 2);
 	ghost_table(A, ghost_rows, ghost_count, B2, nd, (int)(nbr >> 4), nbr, pitch, pp, face_rows);
@@ -322,12 +372,14 @@ __global__ void __launch_bounds__(TMAX, BLOCKS) k_res_cg(const __grid_constant__
 		// Publishes a point of the box's faces (f2, f3: the thread's place in the
 		// i2 and i3 faces) for the neighbours to read after the next fenced sum.
 		auto publish = [&](int c, int d, int f2, int f3, const V &v) {
-			if (c == 0 && lo_c) stl2(faces + f2, v);
-			if (c == hi_c) stl2(faces + f2 + A.nd * n1, v);
-			if (d == 0 && lo_d) stl2(faces + f3 + c * n1, v);
-			if (d == hi_d) stl2(faces + f3 + (B2 + c) * n1, v);
+			const unsigned long long stamp = A.stamp + pub;
+			if (c == 0 && lo_c) faces[f2].put(v, stamp);
+			if (c == hi_c) faces[f2 + A.nd * n1].put(v, stamp);
+			if (d == 0 && lo_d) faces[f3 + c * n1].put(v, stamp);
+			if (d == hi_d) faces[f3 + (B2 + c) * n1].put(v, stamp);
 		};
 		auto publish_all = [&]() {
+			pub++;
 			int f2 = opaque(i1);
 			const int f3 = opaque(own3);
 #pragma unroll
@@ -341,7 +393,7 @@ __global__ void __launch_bounds__(TMAX, BLOCKS) k_res_cg(const __grid_constant__
 			double part[3 * NL];
 			residual(part, true);
 			publish_all();
-			if (!group_sum<3 * NL, true>(g, round, part, Nothing(), [&](int lane, const double (&v)[3 * NL]) {
+			if (!group_sum<3 * NL, !STAMP>(g, round, part, Nothing(), [&](int lane, const double (&v)[3 * NL]) {
 				    if (lane == 0) {
 					    int live = 0;
 #pragma unroll
@@ -393,22 +445,24 @@ __global__ void __launch_bounds__(TMAX, BLOCKS) k_res_cg(const __grid_constant__
 				const int ghosts = *ghost_count;
 				constexpr int HB = 6;
 				for (int h0 = rg; h0 < ghosts; h0 += HB * A.RG) {  // dealt to the row groups
-					V rh[HB];
-					int off[HB];
+					typename FaceT::Got got[HB];
+					int off[HB], from[HB];
 #pragma unroll
 					for (int k = 0; k < HB; k++) {
 						off[k] = -1;
 						if (h0 + k * A.RG >= ghosts) continue;
 						const int2 e = ghost_rows[h0 + k * A.RG];
 						off[k] = e.x + i1;
-						rh[k] = ldl2(faces + e.y + i1);
+						from[k] = e.y + i1;
+						got[k] = faces[from[k]].load();
 					}
 #pragma unroll
 					for (int k = 0; k < HB; k++) {
 						if (off[k] < 0) continue;
+						const V rh = faces[from[k]].get(got[k], A.stamp + pub, g);
 						V p = sp[off[k]];
 #pragma unroll
-						for (int l = 0; l < NL; l++) lane_set(p, l, comb(lane_get(rh[k], l), im, be[l], lane_get(p, l)));
+						for (int l = 0; l < NL; l++) lane_set(p, l, comb(lane_get(rh, l), im, be[l], lane_get(p, l)));
 						sp[off[k]] = p;
 					}
 				}
@@ -533,6 +587,7 @@ __global__ void __launch_bounds__(TMAX, BLOCKS) k_res_cg(const __grid_constant__
 				double v[2 * NL];
 #pragma unroll
 				for (int d = 0; d < 2 * NL; d++) v[d] = 0.0;
+				pub++;
 				if (rows > 0) {
 					S al[NL];
 #pragma unroll
@@ -565,7 +620,7 @@ __global__ void __launch_bounds__(TMAX, BLOCKS) k_res_cg(const __grid_constant__
 						march_rows(update);
 					}
 				}
-				if (!group_sum<2 * NL, true>(g, round, v, Nothing(), [&](int lane, const double (&tot)[2 * NL]) {
+				if (!group_sum<2 * NL, !STAMP>(g, round, v, Nothing(), [&](int lane, const double (&tot)[2 * NL]) {
 #pragma unroll
 					    for (int l = 0; l < NL; l++) {
 						    // Lane 2l: beta; lane 2l + 1: the error and the stop test.
@@ -646,7 +701,7 @@ __global__ void __launch_bounds__(TMAX, BLOCKS) k_res_cg(const __grid_constant__
 					return;  // x_hi complete
 				residual(part, false);
 				publish_all();
-				if (!group_sum<3 * NL, true>(g, round, part, Nothing(), [&](int lane, const double (&tot)[3 * NL]) {
+				if (!group_sum<3 * NL, !STAMP>(g, round, part, Nothing(), [&](int lane, const double (&tot)[3 * NL]) {
 					    if (lane != 0) return;
 					    st.live = 0;
 #pragma unroll
@@ -1314,7 +1369,7 @@ double stream_cycles(int ks, const Geo &g, int lanes, bool fp32) {
 size_t word_bytes(const Plan &p) { return sizeof(Word2) * res_words(p.G) * p.groups; }
 
 size_t edge_bytes(int ks, const Plan &p, const Geo &g) {
-	return 8 * (size_t)kFaces[ks] * (size_t)p.groups * p.G * (2 * p.nd + 2 * p.RG * kShapeC[p.shape]) * g.n1;
+	return (stamped(ks, kShapeC[p.shape]) ? 16 : 8) * (size_t)kFaces[ks] * (size_t)p.groups * p.G * (2 * p.nd + 2 * p.RG * kShapeC[p.shape]) * g.n1;
 }
 
 }  // namespace
@@ -1386,10 +1441,10 @@ static int use_plan(Ctx *c, Resident *R, int units) {
 			return SEDI_ERR_NOMEM;
 		}
 		R->buf_bytes = bytes;
-		// No word may carry a stamp of a launch to come.
-		const cudaError_t e = cudaMemsetAsync(R->buf, 0, bytes, c->stream);
-		if (e != cudaSuccess) return set_cuda_error(c, e, "resident solver");
 	}
+	// No word may carry a stamp of a launch to come, whatever another plan left in its place.
+	const cudaError_t e = cudaMemsetAsync(R->buf, 0, bytes, c->stream);
+	if (e != cudaSuccess) return set_cuda_error(c, e, "resident solver");
 	R->plan = p;
 	R->units = units;
 	return 0;

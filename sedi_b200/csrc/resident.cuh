@@ -50,6 +50,21 @@ struct ResGroup {
 	int fail;                 // a wait of this block ran out
 };
 
+// Waits (bounded) until the word at p is stamped `stamp` and returns it.
+__device__ __forceinline__ Word2 wait2(const Word2 *p, unsigned long long stamp, ResGroup *g) {
+	Word2 w;
+	const long long t0 = clock64();
+	do {
+		w = load2(p);
+		if (w.b != stamp && clock64() - t0 > kResWaitClocks) {
+			g->fail = 1;
+			atomicExch(g->err, 1);
+			break;
+		}
+	} while (w.b != stamp);
+	return w;
+}
+
 // Sums of ND doubles over every thread of the group, in an order fixed by the
 // launch shape; also the group's barrier.  between() runs in every thread
 // after the block's sums are on their way and before the others' are waited
@@ -103,17 +118,7 @@ __device__ __forceinline__ bool group_sum(ResGroup *g, unsigned &round, double (
 			double q[1] = {0.0};
 			if (b < G) {
 				Word2 w = load2(word);
-				if (w.b != stamp) {
-					const long long t0 = clock64();
-					do {
-						w = load2(word);
-						if (w.b != stamp && clock64() - t0 > kResWaitClocks) {
-							g->fail = 1;
-							atomicExch(g->err, 1);
-							break;
-						}
-					} while (w.b != stamp);
-				}
+				if (w.b != stamp) w = wait2(word, stamp, g);
 				q[0] = __longlong_as_double(w.a);
 				if (FENCE) fence_gpu();
 			}
