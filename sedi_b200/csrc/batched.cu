@@ -2475,10 +2475,11 @@ constexpr long long kPairsMinPoints = 1LL << 22;  // smallest grid of the stream
 // vector iM, use the context's march kernels (plain.cu).
 int pairs_alloc(Ctx *c) {
 	c->pairs = nullptr;
-	// Small grids stay on the march kernels: below about 4M points the
-	// single-vector working set sits in the 126 MB L2 and a plane-streaming
-	// block gets too few planes (128^3 CG: 34 probe-solves/s streaming, 43
-	// marching; 256^3: 4.1 against 2.2).
+	// Grids below about 4M points are solved on chip (resident.cu) or, where
+	// they do not fit, by the march kernels: the single-vector working set sits
+	// in the 126 MB L2 and a plane-streaming block gets too few planes (128^3 CG:
+	// 34 probe-solves/s streaming, 43 marching, 122 on chip; 256^3: 4.1 against
+	// 2.2 marching).
 	if (c->g.n1 % 2 != 0 || c->g.n < kPairsMinPoints || !encode_fn()) return 0;
 	Batched *B = new (std::nothrow) Batched();
 	if (!B) return SEDI_ERR_NOMEM;

@@ -1304,7 +1304,9 @@ struct Plan {
 };
 
 // Plan with the smallest estimated time of an iteration of `units` solves, and
-// that time in cycles.  Measured on B200 (FP64, 1.95 GHz): the two reductions,
+// that time in cycles.  Measured on B200 (FP64, 1.95 GHz) before the ghost rows
+// came from a table, which took 1500-6000 cycles off every CG shape alike
+// (16384 points now 32000): the two reductions,
 // ghost rows and launch of each phase take 9000-11000 cycles between blocks;
 // a point adds 1.3 where A p stays in registers (2048 points a block 13600, 8192
 // 20100), 1.65 with two stencil passes (16384: 38000), 1.8 at three rows a
@@ -1473,8 +1475,8 @@ int resident_alloc(Ctx *c, int ks, bool fp32, int lanes, Resident **out) {
 	if (p.shape < 0) return 0;
 	// A pair of FP32 lanes takes 1.6-1.9 times an FP64 lane (conversions for its
 	// FP64 sums).  One right-hand side has no streaming form at these sizes
-	// (its march kernels take 12 us an iteration at 32^3, 47 at 128^3; this 5.6
-	// and 20), a batch does.
+	// (its march kernels take 11.7 us an iteration at 32^3, 47 at 128^3; this 5.5
+	// and 16.4), a batch does.
 	if (fp32) cycles *= 1.8;
 	if (lanes > 1 && cycles > stream_cycles(ks, c->g, lanes, fp32)) return 0;
 	Resident *R = new (std::nothrow) Resident();

@@ -379,9 +379,14 @@ int sedi_slab_sweep(int mode, long n1, long n2, long nloc, double a, double b, d
 int sedi_slab_totals(long n3, const double *plane_part, double *scratch, double *totals, void *stream) {
 	if (n3 < 1 || !plane_part || !scratch || !totals) return SEDI_ERR_ARG;
 	cudaStream_t s = (cudaStream_t)stream;
-	k_slab_totals<<<1, kSlabThreads, 0, s>>>(n3, plane_part, scratch);
+	// Pinned memory is written by the kernel itself: no copy behind it.
+	cudaPointerAttributes at;
+	const bool pinned = cudaPointerGetAttributes(&at, totals) == cudaSuccess && at.type == cudaMemoryTypeHost &&
+	                    at.devicePointer;
+	if (!pinned) cudaGetLastError();
+	k_slab_totals<<<1, kSlabThreads, 0, s>>>(n3, plane_part, pinned ? (double *)at.devicePointer : scratch);
 	if (cudaGetLastError() != cudaSuccess ||
-	    cudaMemcpyAsync(totals, scratch, sizeof(double) * kSlabDots, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+	    (!pinned && cudaMemcpyAsync(totals, scratch, sizeof(double) * kSlabDots, cudaMemcpyDeviceToHost, s) != cudaSuccess) ||
 	    cudaStreamSynchronize(s) != cudaSuccess)
 		return SEDI_ERR_CUDA;
 	return 0;
