@@ -1653,6 +1653,9 @@ struct Batched {
 	double theta = 1.0;  // mixed lanes stop on the FP64 true residual <= theta * tol
 	cudaGraphExec_t graph = nullptr;
 	long long graph_kernels = 0;
+	cudaGraphExec_t other_graph = nullptr;  // iterations of the launch shapes before (start_shape)
+	long long other_kernels = 0;
+	int other_zc[3] = {0, 0, 0};
 	// launch shapes
 	int rbT = 0, rbD = 0;  // lanes per block slice for T and FP64 streams
 	SGeo gT, gD, gT1;
@@ -1770,7 +1773,7 @@ static void tile_for(int rb, int eb, int *P1, int *P2, int kind = 0) {
 }
 
 static void shape(const Geo &g, int R, int rb, int eb, SGeo *sg, dim3 *grid, int nz_force = 0, int kind = 0,
-                  int pfd = -1) {
+                  int pfd = -1, int lanes = 0) {
 	int P1, P2;
 	tile_for(rb, eb, &P1, &P2, kind);
 	const int t1 = (g.n1 + P1 - 1) / P1, t2 = (g.n2 + P2 - 1) / P2;
@@ -1781,8 +1784,9 @@ static void shape(const Geo &g, int R, int rb, int eb, SGeo *sg, dim3 *grid, int
 	// (single-vector CG sweep A at 256^3 on B200: one wave of 128 blocks of
 	// 64 planes, 92 us, beats two waves of 29-plane blocks, 95 us).  Pick the
 	// split with the fewest wave-planes (the last wave counts in full), the
-	// smaller split on ties.
-	const long long per = (long long)t1 * t2 * slices;
+	// smaller split on ties.  Slices past the batch's last lane are padding and
+	// leave at once, so they take no part in the waves.
+	const long long per = (long long)t1 * t2 * (lanes > 0 ? (lanes + rb - 1) / rb : slices);
 	const long long wave = 148LL * SEDI_BLOCKS_PER_SM;
 	long long best = -1;
 	int zc = g.n3, nz = 1;
@@ -1814,6 +1818,56 @@ static void shape(const Geo &g, int R, int rb, int eb, SGeo *sg, dim3 *grid, int
 	sg->tiles1 = t1;
 	sg->pfd = pfd >= 0 ? pfd : (SEDI_STREAM_PFD >= 0 ? SEDI_STREAM_PFD : (zc <= 64 ? 2 : 0));
 	*grid = dim3((unsigned)(t1 * t2), (unsigned)slices, (unsigned)nz);
+}
+
+// Launch shapes for a batch of `lanes` right-hand sides, of the context's R.
+static void shape_for(const Geo &g, Batched *B, int lanes) {
+	const int eb = B->mixed ? 4 : 8;
+	const Tuning &tu = B->tuned;
+	shape(g, B->R, B->rbT, eb, &B->gT, &B->gridT, tu.nz, 0, tu.pfd, lanes);
+	shape(g, B->R, B->rbT, eb, &B->gT1, &B->gridT1, tu.nz, 1, tu.pfd, lanes);
+	shape(g, B->R, B->rbD, 8, &B->gD, &B->gridD, tu.nz, 0, tu.pfd, lanes);
+}
+
+// Blocks of a slice, at most, over every number of lanes: rows of `partials`.
+static size_t most_blocks(const Geo &g, int R, int rbT, int ebT, int rbD, int nz) {
+	size_t most = 0;
+	const int rb = rbT < rbD ? rbT : rbD;
+	for (int lanes = rb; lanes <= R; lanes += rb)
+		for (int k = 0; k < 3; k++) {
+			SGeo sg;
+			dim3 gr;
+			shape(g, R, k == 2 ? rbD : rbT, k == 2 ? 8 : ebT, &sg, &gr, nz, k == 1, -1, lanes);
+			if ((size_t)gr.x * gr.z > most) most = (size_t)gr.x * gr.z;
+		}
+	return most;
+}
+
+static void drop_graphs(Batched *B) {
+	for (cudaGraphExec_t *g : {&B->graph, &B->other_graph}) {
+		if (*g) cudaGraphExecDestroy(*g);
+		*g = nullptr;
+	}
+}
+
+// The shapes of the batch about to start, by its own number of lanes.  By the
+// padded number, blocks of slices that leave at once filled the waves (us an
+// iteration, B200: mixed CG 100^3, 20 lanes in 32: 238, now 195; mixed
+// BiCGStab 90x70x50, 40 in 64: 366 -> 303, 96^3, 18 in 32: 340 -> 278).  The
+// captured iterations hold their shapes; those of the shapes before are kept
+// too, for a last batch that is smaller than the others.
+static void start_shape(Ctx *c, Batched *B, int lanes) {
+	if (B->pairs || B->tuned.nz > 0) return;
+	const int was[3] = {B->gT.zc, B->gT1.zc, B->gD.zc};
+	shape_for(c->g, B, lanes);
+	if (was[0] == B->gT.zc && was[1] == B->gT1.zc && was[2] == B->gD.zc) return;
+	std::swap(B->graph, B->other_graph);
+	std::swap(B->graph_kernels, B->other_kernels);
+	const bool same = B->other_zc[0] == B->gT.zc && B->other_zc[1] == B->gT1.zc && B->other_zc[2] == B->gD.zc;
+	for (int k = 0; k < 3; k++) B->other_zc[k] = was[k];
+	if (same || !B->graph) return;
+	cudaGraphExecDestroy(B->graph);
+	B->graph = nullptr;
 }
 
 template <class C, class Op>
@@ -1912,15 +1966,10 @@ int batched_alloc(Ctx *c) {
 	B->acfg = tu.acfg >= 1 && tu.acfg <= 3 ? tu.acfg : default_form(B->ks, false);
 	B->theta = default_theta(B->ks);
 	if (tu.chunk > 0) B->chunk = tu.chunk;
-	shape(c->g, B->R, B->rbT, ebT, &B->gT, &B->gridT, tu.nz, 0, tu.pfd);
-	shape(c->g, B->R, B->rbT, ebT, &B->gT1, &B->gridT1, tu.nz, 1, tu.pfd);
-	shape(c->g, B->R, B->rbD, 8, &B->gD, &B->gridD, tu.nz, 0, tu.pfd);
+	shape_for(c->g, B, c->batch);
 	const size_t ts = (size_t)ebT;                                  // Krylov field element
 	const size_t xs = B->mixed ? sizeof(float) : sizeof(double);   // x (FP64 form) or x_lo (mixed)
-	const size_t nblkT = (size_t)B->gridT.x * B->gridT.z, nblkD = (size_t)B->gridD.x * B->gridD.z;
-	const size_t nblkT1 = (size_t)B->gridT1.x * B->gridT1.z;
-	size_t nblk = nblkT > nblkD ? nblkT : nblkD;
-	if (nblkT1 > nblk) nblk = nblkT1;
+	const size_t nblk = most_blocks(c->g, B->R, B->rbT, ebT, B->rbD, tu.nz);
 	if (cudaMalloc(&B->x, B->elems * xs) != cudaSuccess || cudaMalloc(&B->r, B->elems * ts) != cudaSuccess ||
 	    cudaMalloc(&B->p0, B->elems * ts) != cudaSuccess || cudaMalloc(&B->p1, B->elems * ts) != cudaSuccess ||
 	    cudaMalloc(&B->b, B->elems * sizeof(double)) != cudaSuccess ||
@@ -2026,16 +2075,7 @@ size_t batched_bytes(int solver, int precision, int batch, long long n1, long lo
 	const Tuning tu = tuning_for(TuneKey{solver, precision, R, n1, n2, n3});
 	int wT = slice_for(R, !mixed, kernel_solver(solver, mixed));
 	if (tu.W > 0 && tu.W <= R && R % tu.W == 0) wT = tu.W;
-	SGeo sT, sD;
-	dim3 gT, gD;
-	shape(g, R, wT, (int)ts, &sT, &gT, tu.nz);
-	shape(g, R, mixed ? mixed_slice_fp64(R) : wT, 8, &sD, &gD, tu.nz);
-	SGeo sT1;
-	dim3 gT1;
-	shape(g, R, wT, (int)ts, &sT1, &gT1, tu.nz, 1);
-	const size_t nblkT = (size_t)gT.x * gT.z, nblkD = (size_t)gD.x * gD.z, nblkT1 = (size_t)gT1.x * gT1.z;
-	size_t nblk = nblkT > nblkD ? nblkT : nblkD;
-	if (nblkT1 > nblk) nblk = nblkT1;
+	const size_t nblk = most_blocks(g, R, wT, (int)ts, mixed ? mixed_slice_fp64(R) : wT, tu.nz);
 	auto up = [](size_t b) { return (b + (2u << 20) - 1) / (2u << 20) * (2u << 20); };
 	const int ks = kernel_solver(solver, mixed);
 	const int nT = 3 + (ks == 3 ? 6 : 0) + (ks == 1 ? 4 : 0);  // r, p0, p1 and the solver's own
@@ -2060,7 +2100,7 @@ static void free_batched(Batched *B) {
 	if (B->lane_host) cudaFreeHost(B->lane_host);
 	if (B->lane_host_int) cudaFreeHost(B->lane_host_int);
 	if (B->ev) cudaEventDestroy(B->ev);
-	if (B->graph) cudaGraphExecDestroy(B->graph);
+	drop_graphs(B);
 	delete B;
 }
 
@@ -2077,7 +2117,7 @@ void batched_free(Ctx *c) {
 	if (B->lane_host) cudaFreeHost(B->lane_host);
 	if (B->lane_host_int) cudaFreeHost(B->lane_host_int);
 	if (B->ev) cudaEventDestroy(B->ev);
-	if (B->graph) cudaGraphExecDestroy(B->graph);
+	drop_graphs(B);
 	delete B;
 	c->batched = nullptr;
 }
@@ -2341,6 +2381,7 @@ struct Impl {
 		g0.nrhs = nrhs;
 		g0.active = 1;
 		*B->g0_host = g0;  // read by the copy below; rewritten only after this batch is over
+		start_shape(c, B, nrhs);
 		BTRY(cudaMemcpyAsync(B->gl, B->g0_host, sizeof(Global), cudaMemcpyHostToDevice, s));
 		enqueue_resid<RBD, PAIRS>(c, B, false);
 		kb_setup_done<<<1, 1, 0, s>>>(B->gl);
@@ -3290,10 +3331,7 @@ int batched_autotune(int solver, int precision, int batch, long long n1, long lo
 		const int chunks[] = {16, 8, 32};
 		int rc = 0;
 		for (int ci = 0; ci < 3 && !rc; ci++) {
-			if (B->graph) {
-				cudaGraphExecDestroy(B->graph);
-				B->graph = nullptr;
-			}
+			drop_graphs(B);
 			B->chunk = chunks[ci];
 			for (int pi = 0; pi < np && !rc; pi++) {
 				if (ci > 0 && periods[pi] != (best.period ? best.period : B->period)) continue;  // chunks at the best period
