@@ -520,6 +520,12 @@ struct OpBase {
 	}
 };
 
+// Two neighbouring lanes in one access.
+template <class T>
+struct alignas(2 * sizeof(T)) Two {
+	T v[2];
+};
+
 // ---------------------------------------------------------------------------
 // Residual sweep (FP64 stream over x and b): r = b - A x (Cg.hpp:119-123).
 // Setup (ru == 0): <b,b>, <r,r> per lane, initial stop test; r stored as TR,
@@ -572,12 +578,14 @@ struct OpResid : OpBase<double> {
 	__device__ void out(long long, long long pidx, int lane, const Vec<double> &, const Vec<double> &ax,
 	                    const Vec<double> *q, const Vec<double> *, const Vec<double> *gv, double (&part)[ND][2]) const {
 		const long long ot = sliced(pidx, lane, WT, npts);  // lanes lane, lane+1 share a TR slice
+		TR rt2[2];
 #pragma unroll
 		for (int e = 0; e < 2; e++) {
 			const double bi = q[0].v[e];
 			const double ri = aadd(bi, -ax.v[e]);  // combine2(1.0, b, -1.0, r, r)
 			const TR rt = (TR)ri;
-			if (!keep[e]) rdst[ot + e] = rt;
+			rt2[e] = rt;
+			if (keep[0] != keep[1] && !keep[e]) rdst[ot + e] = rt;
 			if (xlo) xlo[ot + e] = TR(0);
 			if (ru && solver == 1) {
 				if (restart[e]) rhat[ot + e] = rt;
@@ -589,6 +597,7 @@ struct OpResid : OpBase<double> {
 			}
 			part[1][e] = fma(ri, ri, part[1][e]);
 		}
+		if (!keep[0] && !keep[1]) *reinterpret_cast<Two<TR> *>(rdst + ot) = {{rt2[0], rt2[1]}};  // (one store)
 	}
 	__device__ void fin(int lane, const double *tot, Global *gl, const LaneState &ls) const {
 		// The setup keeps the reference's initial test against tol (:130-134);
@@ -1720,13 +1729,16 @@ __host__ __device__ constexpr int tile_p2(int lg) {
 // 32x16 tile with a 5-stage ring, small enough for two blocks per SM
 // (98 KB each, 64 registers per thread); KIND 3 the 32x32 tile with a
 // 6-stage ring (three planes of TMA lookahead instead of two).
+// KIND 4 is the residual sweep's: with 8-lane FP64 slices a 16x16 tile, two
+// output points per thread and plane barrier instead of one (six stages of
+// 37 KB; a reliable update at 128^3 x 64 lanes 825 -> 701 us).
 template <class T, int RB, int KIND = 0, bool PAIRS = false>
 struct CfgFor {
 	static constexpr int LG = RB * (int)sizeof(T) / 16;
 	static constexpr bool WIDE = (KIND == 1 || KIND == 3) && LG == 1;
 	static constexpr int NSTR = LG != 1 ? 0 : (KIND == 1 ? 4 : (KIND == 2 ? 5 : (KIND == 3 ? 6 : 0)));
 	static constexpr int MINB = (KIND == 2 && LG == 1) ? 2 : 1;
-	typedef Cfg<T, RB, tile_p1(LG), WIDE ? 32 : tile_p2(LG), kThr, NSTR, PAIRS, MINB> type;
+	typedef Cfg<T, RB, tile_p1(LG), WIDE ? 32 : (KIND == 4 && LG == 4 ? 16 : tile_p2(LG)), kThr, NSTR, PAIRS, MINB> type;
 };
 
 static int pick_R(int nrhs, bool mixed) {
@@ -1761,15 +1773,15 @@ static int slice_for(int R, bool fp64, int ks = 0) {
 // FP64 fields of the mixed form (x_hi, b), streamed by the setup and
 // reliable-update residual sweep and the fold: 8-lane slices, so a block's
 // FP32 r (and the fold's x_lo) covers whole 4-lane vectors.  With 2-lane
-// slices (32x16 tiles instead of 16x8) the residual sweep kept its 12.8 ms
-// at 256^3 x 128 (each block wrote half of every FP32 r vector), setup took
+// slices (32x16 tiles instead of 16x8; 16x16 now) the residual sweep kept its
+// 12.8 ms at 256^3 x 128 (each block wrote half of every FP32 r vector), setup took
 // 16.7 against 12.6 ms and the fold 11.1 against 9.6 ms (ncu launch lists).
 static int mixed_slice_fp64(int R) { return slice_for(R, true); }
 
 static void tile_for(int rb, int eb, int *P1, int *P2, int kind = 0) {
 	const int lg = rb * eb / 16;
 	*P1 = tile_p1(lg);
-	*P2 = (kind == 1 && lg == 1) ? 32 : tile_p2(lg);
+	*P2 = (kind == 1 && lg == 1) ? 32 : (kind == 4 && lg == 4 ? 16 : tile_p2(lg));
 }
 
 static void shape(const Geo &g, int R, int rb, int eb, SGeo *sg, dim3 *grid, int nz_force = 0, int kind = 0,
@@ -1826,7 +1838,7 @@ static void shape_for(const Geo &g, Batched *B, int lanes) {
 	const Tuning &tu = B->tuned;
 	shape(g, B->R, B->rbT, eb, &B->gT, &B->gridT, tu.nz, 0, tu.pfd, lanes);
 	shape(g, B->R, B->rbT, eb, &B->gT1, &B->gridT1, tu.nz, 1, tu.pfd, lanes);
-	shape(g, B->R, B->rbD, 8, &B->gD, &B->gridD, tu.nz, 0, tu.pfd, lanes);
+	shape(g, B->R, B->rbD, 8, &B->gD, &B->gridD, tu.nz, 4, tu.pfd, lanes);
 }
 
 // Blocks of a slice, at most, over every number of lanes: rows of `partials`.
@@ -1837,7 +1849,7 @@ static size_t most_blocks(const Geo &g, int R, int rbT, int ebT, int rbD, int nz
 		for (int k = 0; k < 3; k++) {
 			SGeo sg;
 			dim3 gr;
-			shape(g, R, k == 2 ? rbD : rbT, k == 2 ? 8 : ebT, &sg, &gr, nz, k == 1, -1, lanes);
+			shape(g, R, k == 2 ? rbD : rbT, k == 2 ? 8 : ebT, &sg, &gr, nz, k == 2 ? 4 : k, -1, lanes);
 			if ((size_t)gr.x * gr.z > most) most = (size_t)gr.x * gr.z;
 		}
 	return most;
@@ -2042,7 +2054,7 @@ int batched_alloc(Ctx *c) {
 		return k;
 	};
 	bool ok = t_maps(B->mapsT, 0) && t_maps(B->mapsT1, 1);
-	tile_for(B->rbD, 8, &P1, &P2);
+	tile_for(B->rbD, 8, &P1, &P2, 4);
 	ok = ok && make_map(&B->mapsD.m[MD_X_HALO], B->mixed ? (void *)B->xh : B->x, 8, c->g, R, B->rbD, P1 + 2, P2 + 2) &&
 	     make_map(&B->mapsD.m[MD_B_INT], B->b, 8, c->g, R, B->rbD, P1, P2);
 	if (!ok) {
@@ -2125,7 +2137,7 @@ void batched_free(Ctx *c) {
 template <int RBD, bool PAIRS = false>
 static void enqueue_resid(Ctx *c, Batched *B, bool ru) {
 	const int pcg = B->ks == 3 ? 1 : 0;
-	typedef typename CfgFor<double, RBD, 0, PAIRS>::type CD;
+	typedef typename CfgFor<double, RBD, 4, PAIRS>::type CD;
 	cudaStream_t s = c->stream;
 	if (B->mixed) {
 		OpResid<float> op;
