@@ -1473,11 +1473,14 @@ int resident_alloc(Ctx *c, int ks, bool fp32, int lanes, Resident **out) {
 	double cycles = 0.0;
 	const Plan p = plan_for(ks, c->g, fp32 ? (lanes + 1) / 2 : lanes, sms, shared, &cycles);
 	if (p.shape < 0) return 0;
-	// A pair of FP32 lanes takes 1.6-1.9 times an FP64 lane (conversions for its
-	// FP64 sums).  One right-hand side has no streaming form at these sizes
-	// (its march kernels take 11.7 us an iteration at 32^3, 47 at 128^3; this 5.5
-	// and 16.4), a batch does.
-	if (fp32) cycles *= 1.8;
+	// A pair of FP32 lanes takes 1.45-1.7 times what the estimate says of an FP64
+	// lane (conversions for its FP64 sums, less since the ghost table); at 1.6 no
+	// measured batch goes on chip that is slower there (us an iteration, on chip and
+	// streaming: 80^3 x 32 110 / 133; 96^3 x 16 105 / 99, 96^3 x 32 208 / 168,
+	// 128^3 x 16 230 / 201; 64^3 x 64, 107 / 115, and 80^3 x 64, 221 / 240, stream).  One right-hand side has no streaming
+	// form at these sizes (its march kernels take 11.7 us an iteration at 32^3, 47
+	// at 128^3; this 5.5 and 16.4), a batch does.
+	if (fp32) cycles *= 1.6;
 	if (lanes > 1 && cycles > stream_cycles(ks, c->g, lanes, fp32)) return 0;
 	Resident *R = new (std::nothrow) Resident();
 	if (!R) return SEDI_ERR_NOMEM;
