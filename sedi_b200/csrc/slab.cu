@@ -14,8 +14,8 @@
 // Dot products are returned per plane, each summed in a fixed order that
 // depends only on n1 and n2 (the plane is cut into kSlabChunks row chunks, a
 // cluster of kSlabSplit blocks each, then the chunks are added in a fixed tree), so a plane's partial
-// sum is the same whichever rank holds the plane; the host adds the planes
-// in global order.  The solution therefore does not depend on the number of
+// sum is the same whichever rank holds the plane; the planes are then added in
+// an order fixed by their number (k_slab_totals).  The solution therefore does not depend on the number of
 // slabs, bit for bit.  Elementwise values round as the reference's
 // (operator by operator, no FMA contraction), like the single-vector form:
 // a stencil input the reference stores (u = r .* iM, m = w .* iM, p_hat,
@@ -137,6 +137,11 @@ __global__ void __cluster_dims__(kSlabSplit, 1, 1) __launch_bounds__(kSlabThread
 #pragma unroll
 	for (int d = 0; d < ND; d++) v[d] = 0.0;
 	const double iM = a.iM;
+	// A block's shared memory may be written by its cluster only once it is known
+	// to run: every thread says so here and waits for the others' word behind the
+	// rows, where it has long arrived.
+	cg::cluster_group cluster = cg::this_cluster();
+	if (mode_dots(MODE) > 0) cluster.barrier_arrive();
 	// Rows of the chunk, each by tpr threads (row_threads), the block's other
 	// threads on the next rows.  Not unrolled: these sweeps hide latency with
 	// resident warps, and unrolling by 4 cost more in occupancy (registers) than
@@ -237,7 +242,7 @@ __global__ void __cluster_dims__(kSlabSplit, 1, 1) __launch_bounds__(kSlabThread
 	block_total<ND>(v);
 	// The chunk's blocks hand their sums to the first of them, which adds them in order.
 	__shared__ double part[kSlabSplit][ND];
-	cg::cluster_group cluster = cg::this_cluster();
+	cluster.barrier_wait();
 	if (threadIdx.x == 0)
 #pragma unroll
 		for (int d = 0; d < ND; d++) cluster.map_shared_rank(&part[c % kSlabSplit][d], 0)[0] = v[d];
