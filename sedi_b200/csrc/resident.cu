@@ -25,6 +25,7 @@
 #include <vector>
 
 #include "resident.cuh"
+#include "resident_room.h"
 #include "sedi_internal.h"
 
 namespace sedi {
@@ -1388,15 +1389,12 @@ struct Resident {
 	unsigned long long launch = 0;
 	int device = 0, sms = 0;
 	cudaEvent_t done = nullptr;  // after the latest launch
-	int held = 0;                // SMs of that launch while it may run
+	RoomUse use;                 // of that launch while it may run
 };
 
-// Launches that may be running, oldest first.  The blocks of a launch wait for
-// one another, so all of them must find room: two launches that each hold a
-// part of the GPU and wait for the rest would never end.  A new launch
-// therefore waits (on its stream) for the oldest ones until those it may
-// overlap and itself need no more SMs than there are.  Other kernels end by
-// themselves.  One entry per context, taken out when the context goes.
+// Launches that may be running, oldest first (resident_room.h says which of
+// them a new one waits for).  One entry per context, taken out when the context
+// goes.
 static std::mutex g_running_mu;
 static std::vector<Resident *> g_running;
 
@@ -1558,10 +1556,14 @@ int resident_launch(Ctx *c, Resident *R, const ResIO &io) {
 	a.hist = io.hist;
 	a.err = io.err;
 	void *args[] = {&a};
-	const int blocks = groups * p.G, per_sm = kShapeB[p.shape], need = p.G > 1 ? (blocks + per_sm - 1) / per_sm : 0;
+	const int blocks = groups * p.G;
+	const RoomUse use = room_use(blocks, p.G, R->sms);
 	std::lock_guard<std::mutex> lk(g_running_mu);
+	// A context's launch has ended when its next one comes: a call waits for its
+	// stream, an estimate's next step for its event.
 	running_remove(R);
-	int held = need;
+	std::vector<Resident *> others;
+	std::vector<RoomUse> uses;
 	for (size_t i = 0; i < g_running.size();) {
 		Resident *const o = g_running[i];
 		if (o->device == R->device) {
@@ -1569,22 +1571,22 @@ int resident_launch(Ctx *c, Resident *R, const ResIO &io) {
 				g_running.erase(g_running.begin() + (long)i);
 				continue;
 			}
-			held += o->held;
+			others.push_back(o);
+			uses.push_back(o->use);
 		}
 		i++;
 	}
-	for (size_t i = 0; need > 0 && held > R->sms && i < g_running.size(); i++) {
-		Resident *const o = g_running[i];
-		if (o->device != R->device) continue;
-		const cudaError_t w = cudaStreamWaitEvent(c->stream, o->done, 0);
+	const std::vector<char> wait = room_waits(uses, use, R->sms);
+	for (size_t i = 0; i < others.size(); i++) {
+		if (!wait[i]) continue;
+		const cudaError_t w = cudaStreamWaitEvent(c->stream, others[i]->done, 0);
 		if (w != cudaSuccess) return set_cuda_error(c, w, "resident solver launch");
-		held -= o->held;
 	}
 	cudaError_t e = cudaLaunchCooperativeKernel((const void *)kernel_for(R->ks, R->fp32, R->unit, p.shape), dim3((unsigned)blocks),
 	                                            dim3((unsigned)p.T), args, p.smem, c->stream);
-	if (e == cudaSuccess && need > 0) {
+	if (e == cudaSuccess) {
 		e = cudaEventRecord(R->done, c->stream);
-		R->held = need;
+		R->use = use;
 		g_running.push_back(R);
 	}
 	if (e != cudaSuccess) return set_cuda_error(c, e, "resident solver launch");
