@@ -708,6 +708,14 @@ struct OpCgA : OpBase<T> {
 #pragma unroll
 		for (int e = 0; e < V; e++) beta[e] = (T)ls.beta[lane + e];
 	}
+	// A lane that stopped on an odd iteration has its x step taken by the next
+	// sweep B, which also adds alpha = 0 times the direction this sweep writes:
+	// left out, that would be whatever an earlier batch had there (0 x NaN).
+	__device__ bool slice_live(const Global *gl, const LaneState &ls, int lane0, int nl) const {
+		for (int l = lane0; l < lane0 + nl; l++)
+			if (!ls.done[l] || (!(gl->iter & 1) && ls.xa[l] != 0.0)) return true;
+		return false;
+	}
 	__device__ bool raw_center() const { return first; }  // <r,u> is only needed on iteration 1
 	__device__ int src_map(int s) const { return s == 0 ? MT_R_HALO : ((it & 1) ? MT_P0_HALO : MT_P1_HALO); }
 	__device__ int q_map(int) const { return 0; }
