@@ -512,11 +512,12 @@ int plain_alloc(Ctx *c) {
 	const size_t sweep_blocks = (size_t)l.grid.x * l.grid.y * l.grid.z;
 	SEDI_TRY(cudaMalloc(&c->partials, sizeof(double) * kMaxDots * (sweep_blocks > (size_t)c->nblocks ? sweep_blocks : (size_t)c->nblocks)));
 	SEDI_TRY(cudaMalloc(&c->ticket, sizeof(unsigned)));
-	SEDI_TRY(cudaMemsetAsync(c->ticket, 0, sizeof(unsigned), c->stream));  // ordered before the context's kernels
-	SEDI_TRY(cudaStreamSynchronize(c->stream));
 	SEDI_TRY(cudaMalloc(&c->st, sizeof(SolveState)));
-	SEDI_TRY(cudaMemsetAsync(c->st, 0, sizeof(SolveState), c->stream));
 	SEDI_TRY(cudaMallocHost(&c->st_host, sizeof(SolveState)));
+	// Done before a solve on the caller's stream (sedi_set_stream) may use them.
+	SEDI_TRY(cudaMemsetAsync(c->ticket, 0, sizeof(unsigned), c->stream));
+	SEDI_TRY(cudaMemsetAsync(c->st, 0, sizeof(SolveState), c->stream));
+	SEDI_TRY(cudaStreamSynchronize(c->stream));
 	c->hist_cap = 0;
 	c->hist = nullptr;
 	c->chunk_iters = 16;
