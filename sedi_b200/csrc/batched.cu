@@ -1990,8 +1990,15 @@ int batched_alloc(Ctx *c) {
 	const size_t ts = (size_t)ebT;                                  // Krylov field element
 	const size_t xs = B->mixed ? sizeof(float) : sizeof(double);   // x (FP64 form) or x_lo (mixed)
 	const size_t nblk = most_blocks(c->g, B->R, B->rbT, ebT, B->rbD, tu.nz);
+	// The on-chip solver's buffer lies behind p1, which it does not use.  Its rule
+	// takes the padded lanes, like the buffer: a batch that fits them runs the same
+	// way on every context of that many.
+	size_t room = 0;
+	int rrc = resident_alloc(c, B->ks, B->mixed, B->R, c->batch, &B->res, &room);
+	if (rrc) return rrc;
+	const size_t p1_bytes = (B->elems * ts + 255) / 256 * 256;
 	if (cudaMalloc(&B->x, B->elems * xs) != cudaSuccess || cudaMalloc(&B->r, B->elems * ts) != cudaSuccess ||
-	    cudaMalloc(&B->p0, B->elems * ts) != cudaSuccess || cudaMalloc(&B->p1, B->elems * ts) != cudaSuccess ||
+	    cudaMalloc(&B->p0, B->elems * ts) != cudaSuccess || cudaMalloc(&B->p1, p1_bytes + room) != cudaSuccess ||
 	    cudaMalloc(&B->b, B->elems * sizeof(double)) != cudaSuccess ||
 	    (B->mixed && cudaMalloc(&B->xh, B->elems * sizeof(double)) != cudaSuccess) ||
 	    cudaMalloc(&B->partials, sizeof(double) * nblk * kMaxDots * B->R) != cudaSuccess ||
@@ -2071,8 +2078,7 @@ int batched_alloc(Ctx *c) {
 	}
 	B->g0_host = B->gl_host + 1;
 	B->lane_res.assign(B->R, 0);
-	const int rrc = resident_alloc(c, B->ks, B->mixed, B->R, &B->res);
-	if (rrc) return rrc;
+	if (B->res && (rrc = resident_bind(c, B->res, (char *)B->p1 + p1_bytes))) return rrc;
 	bind_impl(B);
 	// The zero-fills must be complete before a caller stream (sedi_set_stream) uses the buffers.
 	if (cudaStreamSynchronize(c->stream) != cudaSuccess) return set_cuda_error(c, cudaGetLastError(), "batched_alloc");
@@ -2099,10 +2105,16 @@ size_t batched_bytes(int solver, int precision, int batch, long long n1, long lo
 	auto up = [](size_t b) { return (b + (2u << 20) - 1) / (2u << 20) * (2u << 20); };
 	const int ks = kernel_solver(solver, mixed);
 	const int nT = 3 + (ks == 3 ? 6 : 0) + (ks == 1 ? 4 : 0);  // r, p0, p1 and the solver's own
-	size_t total = nT * up(elems * ts) + up(elems * xs) + up(elems * 8) * (mixed ? 2 : 1);
+	// The on-chip solver's buffer, behind p1: the most of any solver, so that jobs
+	// on a grid differ by their fields.
+	size_t room = 0;
+	for (int k = 1; k <= 3; k++) {
+		const size_t b = resident_bytes(k, mixed, R, g);
+		if (b > room) room = b;
+	}
+	size_t total = (nT - 1) * up(elems * ts) + up((elems * ts + 255) / 256 * 256 + room) + up(elems * xs) + up(elems * 8) * (mixed ? 2 : 1);
 	total += up(sizeof(double) * nblk * kMaxDots * R) + 3 * up(1) + up(sizeof(double) * kLaneDoubles * R) +
 	         up(sizeof(int) * 5 * R) + 2 * up(sizeof(double) * g.n);
-	if (g.n1 <= 512 && g.n <= (1 << 22)) total += 12 * up(1);  // the resident solver's face rows and reduction words
 	return total;
 }
 

@@ -501,8 +501,12 @@ int plain_alloc(Ctx *c) {
 	c->nblocks = blocks_for(c->g.n);
 	double **vecs[] = {&c->x, &c->b, &c->iM, &c->r, &c->rhat, &c->p[0], &c->p[1], &c->v[0], &c->v[1],
 	                   &c->w[0], &c->w[1], &c->u, &c->q, &c->s, &c->z, &c->t_acc, &c->q_acc};
+	size_t room = 0;  // of the resident solver, behind z
+	int rc = resident_alloc(c, c->solver, false, 1, 1, &c->res, &room);
+	if (rc) return rc;
+	const size_t z_bytes = (bytes + 255) / 256 * 256;
 	for (double **pp : vecs) {
-		if (cudaMalloc(pp, bytes) != cudaSuccess) {
+		if (cudaMalloc(pp, pp == &c->z ? z_bytes + room : bytes) != cudaSuccess) {
 			cudaGetLastError();
 			c->error = "device allocation failed";
 			return SEDI_ERR_NOMEM;
@@ -517,12 +521,12 @@ int plain_alloc(Ctx *c) {
 	// Done before a solve on the caller's stream (sedi_set_stream) may use them.
 	SEDI_TRY(cudaMemsetAsync(c->ticket, 0, sizeof(unsigned), c->stream));
 	SEDI_TRY(cudaMemsetAsync(c->st, 0, sizeof(SolveState), c->stream));
+	if (c->res && (rc = resident_bind(c, c->res, (char *)c->z + z_bytes))) return rc;
 	SEDI_TRY(cudaStreamSynchronize(c->stream));
 	c->hist_cap = 0;
 	c->hist = nullptr;
 	c->chunk_iters = 16;
-	const int rc = resident_alloc(c, c->solver, false, 1, &c->res);
-	return rc ? rc : pairs_alloc(c);
+	return pairs_alloc(c);
 }
 
 void plain_free(Ctx *c) {

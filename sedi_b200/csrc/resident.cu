@@ -1304,8 +1304,16 @@ struct Plan {
 	size_t smem = 0;
 };
 
+// Device memory of a launch: the groups' reduction words, then the boxes' faces.
+size_t word_bytes(int G, int groups) { return sizeof(Word2) * res_words(G) * groups; }
+size_t buffer_bytes(int ks, int shape, int G, int groups, int nd, int RG, int n1) {
+	return word_bytes(G, groups) +
+	       (stamped(ks, kShapeC[shape]) ? 16 : 8) * (size_t)kFaces[ks] * groups * G * (2 * nd + 2 * RG * kShapeC[shape]) * n1;
+}
+
 // Plan with the smallest estimated time of an iteration of `units` solves, and
-// that time in cycles.  Measured on B200 (FP64, 1.95 GHz) before the ghost rows
+// that time in cycles; *most grows to the buffer of any plan for at most `units`
+// solves.  Measured on B200 (FP64, 1.95 GHz) before the ghost rows
 // came from a table, which took 1500-6000 cycles off every CG shape alike
 // (16384 points now 32000): the two reductions,
 // ghost rows and launch of each phase take 9000-11000 cycles between blocks;
@@ -1315,7 +1323,7 @@ struct Plan {
 // Pipelined CG: 256 points a block 7700, 2048 10400, 4096 14000; BiCGStab: 512
 // points 19000, 2048 24000, 4096 29000, 6144 (x in L2) 52000; pipelined CG's
 // 6144 points (two or three fields in L2) 27700.
-Plan plan_for(int ks, const Geo &g, int units, int sms, size_t smem_max, double *cycles) {
+Plan plan_for(int ks, const Geo &g, int units, int sms, size_t smem_max, double *cycles, size_t *most = nullptr) {
 	constexpr double kPoint[kCgShapes] = {1.3, 1.3, 1.3, 1.65, 1.8, 3.2};
 	constexpr double kSync[4] = {0.0, 16000.0, 9000.0, 6000.0}, kPointOf[4] = {0.0, 2.9, 0.0, 1.6};  // by solver id
 	Plan best;
@@ -1334,6 +1342,10 @@ Plan plan_for(int ks, const Geo &g, int units, int sms, size_t smem_max, double 
 				const size_t smem = ghosted + nsm * own;
 				if (G > slots || smem * kShapeB[sh] > smem_max) continue;
 				const int groups = units < slots / (int)G ? units : slots / (int)G;
+				if (most) {
+					const size_t bytes = buffer_bytes(ks, sh, (int)G, groups, nd, RG, g.n1);
+					if (bytes > *most) *most = bytes;
+				}
 				const double point = ks == SEDI_CG ? kPoint[sh < kCgShapes ? sh : 0] : kPointOf[ks] * (ks == SEDI_BICGSTAB && nd > 8 ? 1.7 : 1.0);
 				const double deep = ks != SEDI_CG && nd > 4 ? 1500.0 : 0.0;  // the deeper kernels' start-up
 				const double cost = ((G > 1 ? kSync[ks] + 15.0 * G : kSync[ks] / 3.0) + deep +
@@ -1369,22 +1381,19 @@ double stream_cycles(int ks, const Geo &g, int lanes, bool fp32) {
 	return 1950.0 * (kLaunch[ks] + kWords[ks] * (fp32 ? 4.0 : 8.0) * (double)g.n * lanes * std::sqrt(over) / 5.9e6);
 }
 
-size_t word_bytes(const Plan &p) { return sizeof(Word2) * res_words(p.G) * p.groups; }
-
-size_t edge_bytes(int ks, const Plan &p, const Geo &g) {
-	return (stamped(ks, kShapeC[p.shape]) ? 16 : 8) * (size_t)kFaces[ks] * (size_t)p.groups * p.G * (2 * p.nd + 2 * p.RG * kShapeC[p.shape]) * g.n1;
-}
-
 }  // namespace
 
 struct Resident {
-	Plan plan;
-	int units = 0;          // solves the plan is for
+	struct {
+		Plan plan;
+		int units = 0;      // solves the plan is for
+	} plans[2];             // a last batch may be smaller than the others
+	int now = 0;            // the one whose launch the buffer is laid out for
 	int ks = 0;
 	bool fp32 = false, unit = false;
 	size_t shared = 0;      // shared memory of a block, at most
 	bool ready[kShapes] = {};
-	void *buf = nullptr;    // the groups' reduction words, then the boxes' faces
+	void *buf = nullptr;    // the owner's memory, enough for every plan
 	size_t buf_bytes = 0;
 	unsigned long long launch = 0;
 	int device = 0, sms = 0;
@@ -1406,71 +1415,75 @@ static void running_remove(Resident *R) {
 		}
 }
 
+// Makes plan p's kernel ready; false where it cannot run.
+static bool kernel_ready(Resident *R, const Plan &p) {
+	if (R->ready[p.shape]) return true;
+	const void *const k = (const void *)kernel_for(R->ks, R->fp32, R->unit, p.shape);
+	int per_sm = 0;
+	// (The attribute is the kernel's, whoever launches it: its largest use.)
+	if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(R->shared / kShapeB[p.shape])) !=
+	        cudaSuccess ||
+	    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kShapeT[p.shape], R->shared / kShapeB[p.shape]) !=
+	        cudaSuccess ||
+	    per_sm < kShapeB[p.shape]) {
+		cudaGetLastError();
+		return false;
+	}
+	return R->ready[p.shape] = true;
+}
+
 // Plan for `units` solves, chosen by their number and the grid alone (so a
 // result does not depend on the context's room for more): 10 FP64 solves of
 // 58^3 on a plan for 16 ran as 9 groups and one more round.  The one in use
-// stays where the kernel of a better one cannot run.
+// stays where the kernel of a better one cannot run.  Two are kept, and the
+// buffer holds any, so that no call allocates and batches whose size alternates
+// do not search again (1-110 us).
 static int use_plan(Ctx *c, Resident *R, int units) {
-	if (units == R->units) return 0;
-	double cycles = 0.0;
-	const Plan p = plan_for(R->ks, c->g, units, R->sms, R->shared, &cycles);
-	if (p.shape < 0) return 0;
-	if (!R->ready[p.shape]) {
-		const void *const k = (const void *)kernel_for(R->ks, R->fp32, R->unit, p.shape);
-		int per_sm = 0;
-		// (The attribute is the kernel's, whoever launches it: its largest use.)
-		if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(R->shared / kShapeB[p.shape])) !=
-		        cudaSuccess ||
-		    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kShapeT[p.shape], R->shared / kShapeB[p.shape]) !=
-		        cudaSuccess ||
-		    per_sm < kShapeB[p.shape]) {
-			cudaGetLastError();
-			return 0;
-		}
-		R->ready[p.shape] = true;
-	}
-	const size_t bytes = word_bytes(p) + edge_bytes(R->ks, p, c->g);
-	if (bytes > R->buf_bytes) {
-		if (R->buf) cudaFree(R->buf);
-		R->buf = nullptr;
-		R->buf_bytes = 0;
-		R->units = 0;
-		if (cudaMalloc(&R->buf, bytes) != cudaSuccess) {
-			cudaGetLastError();
-			c->error = "device allocation failed (resident solver)";
-			return SEDI_ERR_NOMEM;
-		}
-		R->buf_bytes = bytes;
+	if (units == R->plans[R->now].units) return 0;
+	const int other = R->now ^ 1;
+	if (units != R->plans[other].units) {
+		double cycles = 0.0;
+		const Plan p = plan_for(R->ks, c->g, units, R->sms, R->shared, &cycles);
+		if (p.shape < 0 || !kernel_ready(R, p)) return 0;
+		R->plans[other].plan = p;
+		R->plans[other].units = units;
 	}
 	// No word may carry a stamp of a launch to come, whatever another plan left in its place.
-	const cudaError_t e = cudaMemsetAsync(R->buf, 0, bytes, c->stream);
+	const Plan &p = R->plans[other].plan;
+	const cudaError_t e =
+	    cudaMemsetAsync(R->buf, 0, buffer_bytes(R->ks, p.shape, p.G, p.groups, p.nd, p.RG, c->g.n1), c->stream);
 	if (e != cudaSuccess) return set_cuda_error(c, e, "resident solver");
-	R->plan = p;
-	R->units = units;
+	R->now = other;
 	return 0;
 }
 
-// A resident solver for `lanes` right-hand sides of the context's grid; *out
-// stays null where the grid or the device does not take one (the streaming
-// and march kernels serve those).
-int resident_alloc(Ctx *c, int ks, bool fp32, int lanes, Resident **out) {
-	*out = nullptr;
-	if (ks != SEDI_CG && fp32) return 0;
-	if (c->g.n1 > 512 || c->g.n > (1 << 22)) return 0;  // no box shape takes them
-	int sms = 0, coop = 0, smem_max = 0;
-	const bool unit = c->k.b == 1.0 && c->k.c == 1.0;
-	if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device) != cudaSuccess ||
-	    cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, c->device) != cudaSuccess ||
-	    cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device) != cudaSuccess || !coop) {
+// What a block may use and the blocks at once, of the current device; of a B200
+// where there is none.
+static bool resident_limits(int device, int *sms, size_t *shared) {
+	int coop = 1, smem_max = 232448;
+	*sms = 148;
+	if (device >= 0 && (cudaDeviceGetAttribute(sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
+	                    cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device) != cudaSuccess ||
+	                    cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, device) != cudaSuccess)) {
 		cudaGetLastError();
-		return 0;
+		return false;
 	}
 	// Beside the static arrays and what the system keeps, for up to two blocks of an SM.
-	const size_t shared = (size_t)smem_max - 2 * (sizeof(ResGroup) + sizeof(CgState<2>) + 1024);
-	if (sms > kResMaxBlocks / 2) sms = kResMaxBlocks / 2;
+	*shared = (size_t)smem_max - 2 * (sizeof(ResGroup) + sizeof(CgState<2>) + 1024);
+	if (*sms > kResMaxBlocks / 2) *sms = kResMaxBlocks / 2;
+	return coop != 0;
+}
+
+// Whether `lanes` right-hand sides of a grid are solved on chip; then *most is
+// the buffer that any number of them up to that needs.
+static bool resident_takes(int ks, bool fp32, int lanes, const Geo &g, int sms, size_t shared, size_t *most) {
+	*most = 0;
+	if (ks != SEDI_CG && fp32) return false;
+	if (g.n1 > 512 || g.n > (1 << 22)) return false;  // no box shape takes them
 	double cycles = 0.0;
-	const Plan p = plan_for(ks, c->g, fp32 ? (lanes + 1) / 2 : lanes, sms, shared, &cycles);
-	if (p.shape < 0) return 0;
+	const Plan p = plan_for(ks, g, fp32 ? (lanes + 1) / 2 : lanes, sms, shared, &cycles, most);
+	if (p.shape < 0) return false;
+	if (lanes == 1) *most = buffer_bytes(ks, p.shape, p.G, p.groups, p.nd, p.RG, g.n1);  // (one plan)
 	// A pair of FP32 lanes takes 1.45-1.7 times what the estimate says of an FP64
 	// lane (conversions for its FP64 sums, less since the ghost table); at 1.6 no
 	// measured batch goes on chip that is slower there (us an iteration, on chip and
@@ -1479,23 +1492,60 @@ int resident_alloc(Ctx *c, int ks, bool fp32, int lanes, Resident **out) {
 	// form at these sizes (its march kernels take 11.7 us an iteration at 32^3, 47
 	// at 128^3; this 5.5 and 16.4), a batch does.
 	if (fp32) cycles *= 1.6;
-	if (lanes > 1 && cycles > stream_cycles(ks, c->g, lanes, fp32)) return 0;
+	return lanes <= 1 || cycles <= stream_cycles(ks, g, lanes, fp32);
+}
+
+// Buffer of a resident solver (see resident_alloc), 0 where there is none.
+size_t resident_bytes(int ks, bool fp32, int lanes, const Geo &g) {
+	int device = -1, count = 0, sms = 0;
+	size_t shared = 0, most = 0;
+	if (cudaGetDeviceCount(&count) != cudaSuccess || count == 0 || cudaGetDevice(&device) != cudaSuccess) {
+		cudaGetLastError();
+		device = -1;
+	}
+	return resident_limits(device, &sms, &shared) && resident_takes(ks, fp32, lanes, g, sms, shared, &most) ? most : 0;
+}
+
+// A resident solver for up to `lanes` right-hand sides of the context's grid,
+// planned for `batch` of them; *out stays null where the grid or the device does
+// not take one (the streaming and march kernels serve those).  The caller gives
+// it *bytes of device memory, 16-byte aligned, with resident_bind: as the tail of
+// a vector, since an allocation of its own took 0.4 ms of a context's creation.
+int resident_alloc(Ctx *c, int ks, bool fp32, int lanes, int batch, Resident **out, size_t *bytes) {
+	*out = nullptr;
+	*bytes = 0;
+	int sms = 0;
+	size_t shared = 0, most = 0;
+	if (!resident_limits(c->device, &sms, &shared) || !resident_takes(ks, fp32, lanes, c->g, sms, shared, &most)) return 0;
 	Resident *R = new (std::nothrow) Resident();
 	if (!R) return SEDI_ERR_NOMEM;
 	R->ks = ks;
 	R->fp32 = fp32;
-	R->unit = unit;
+	R->unit = c->k.b == 1.0 && c->k.c == 1.0;
 	R->shared = shared;
 	R->device = c->device;
 	R->sms = sms;
-	const int rc = use_plan(c, R, fp32 ? (lanes + 1) / 2 : lanes);
-	if (rc || R->plan.shape < 0 || cudaEventCreateWithFlags(&R->done, cudaEventDisableTiming) != cudaSuccess) {
+	R->buf_bytes = most;
+	const int units = fp32 ? (batch + 1) / 2 : batch;
+	double cycles = 0.0;
+	R->plans[0].plan = plan_for(ks, c->g, units, sms, shared, &cycles);
+	R->plans[0].units = units;
+	if (R->plans[0].plan.shape < 0 || !kernel_ready(R, R->plans[0].plan) ||
+	    cudaEventCreateWithFlags(&R->done, cudaEventDisableTiming) != cudaSuccess) {
 		cudaGetLastError();
 		resident_free(R);
-		return rc;
+		return 0;
 	}
 	*out = R;
-	return cudaStreamSynchronize(c->stream) == cudaSuccess ? 0 : set_cuda_error(c, cudaGetLastError(), "resident_alloc");
+	*bytes = most;
+	return 0;
+}
+
+// The owner's memory for R; zeroed on the context's stream, for which the caller waits.
+int resident_bind(Ctx *c, Resident *R, void *buf) {
+	R->buf = buf;
+	const cudaError_t e = cudaMemsetAsync(buf, 0, R->buf_bytes, c->stream);
+	return e == cudaSuccess ? 0 : set_cuda_error(c, e, "resident solver");
 }
 
 void resident_free(Resident *R) {
@@ -1505,7 +1555,6 @@ void resident_free(Resident *R) {
 		running_remove(R);
 	}
 	if (R->done) cudaEventDestroy(R->done);
-	if (R->buf) cudaFree(R->buf);
 	delete R;
 }
 
@@ -1515,7 +1564,7 @@ int resident_launch(Ctx *c, Resident *R, const ResIO &io) {
 	if (units < 1) return 0;
 	const int rc = use_plan(c, R, units);
 	if (rc) return rc;
-	const Plan &p = R->plan;
+	const Plan &p = R->plans[R->now].plan;
 	const int groups = units < p.groups ? units : p.groups;
 	ResArgs a;
 	a.n1 = c->g.n1;
@@ -1538,7 +1587,7 @@ int resident_launch(Ctx *c, Resident *R, const ResIO &io) {
 	a.x = io.x;
 	a.xlo = (float2 *)io.xlo;
 	a.words = (Word2 *)R->buf;
-	a.edge = (char *)R->buf + word_bytes(p);
+	a.edge = (char *)R->buf + word_bytes(p.G, p.groups);
 	a.stamp = ++R->launch << 36;
 	a.tol = io.tol;
 	a.tol_in = io.tol_in;

@@ -158,7 +158,9 @@ struct ResIO {
 	double *hist;
 	int *err;
 };
-int resident_alloc(Ctx *c, int ks, bool fp32, int lanes, Resident **out);
+size_t resident_bytes(int ks, bool fp32, int lanes, const Geo &g);
+int resident_alloc(Ctx *c, int ks, bool fp32, int lanes, int batch, Resident **out, size_t *bytes);
+int resident_bind(Ctx *c, Resident *R, void *buf);
 void resident_free(Resident *R);
 int resident_launch(Ctx *c, Resident *R, const ResIO &io);
 

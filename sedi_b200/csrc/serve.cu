@@ -21,11 +21,12 @@
 //
 // A job's lane count depends only on the job and the server's per-job byte
 // cap, never on the load, and every reduction runs in a fixed order, so a
-// job's result is the same alone and in any mix.  A context's launch shapes
-// depend only on its padded lane count, so a job whose probes fit one batch
-// may run on any context of its padded lane count with room for them (new
-// contexts are created with every padded lane usable); a job of several
-// batches runs only on contexts of its own batch size.
+// job's result is the same alone and in any mix.  A batch's form and launch
+// shapes depend only on its context's padded lane count and on its own number of
+// right-hand sides, so a job whose probes fit one batch may run on any context of
+// its padded lane count with room for them (new contexts are created with every
+// padded lane usable); a job of several batches runs only on contexts of its own
+// batch size.
 #include <chrono>
 #include <cmath>
 #include <cstring>
