@@ -148,7 +148,10 @@ int sedi_set_stream(sedi_ctx *ctx, void *stream);
  * slots).  The buffers' contents are scratch afterwards.  Returns 0 or error.
  * A single-vector FP64 context (batch 1) times its streaming sweeps (names
  * ending in _sv), which serve grids with n1 even and at least 2^22 points;
- * SEDI_ERR_UNSUPPORTED for other grids, which use column-march kernels.
+ * SEDI_ERR_UNSUPPORTED for other grids, which are solved on chip in one launch
+ * or by column-march kernels.  A batched context always times its sweeps, also
+ * where its solves run on chip (grids whose Krylov vectors fit there) and launch
+ * none of them.
  * CG lists three kernels: cg_a every iteration, and its second sweep in two
  * forms that alternate, cg_b on odd iterations (r only) and cg_bx on even
  * ones (the x steps of both iterations).
@@ -361,7 +364,10 @@ int sedi_server_stats(const sedi_server *srv, double *peak_bytes, double *budget
  * distance), narrow-sweep form; *score_ms (optional)
  * = the winning estimate time (flags & 1) or the sweep time of one
  * iteration (CG's two parity forms of sweep B count half each).  Needs
- * device memory for one such context at a time.
+ * device memory for one such context at a time.  Where the solves run on chip
+ * the choices of the sweeps act on nothing: only the reliable-update period is
+ * measured, the others are the built-in ones, and *score_ms without flags & 1 is
+ * the time of one iteration of `batch` solves.
  */
 int sedi_autotune(int solver, int precision, int batch, long n1, long n2, long n3, int maxiter, double tol,
                   uint32_t seed, int flags, int *choice, double *score_ms);
@@ -373,8 +379,8 @@ int sedi_autotune(int solver, int precision, int batch, long n1, long n2, long n
  * that of the prefetch distance) sets it again at start-up.  With
  * SEDI_PREC_FP64 and batch 1 it sets the single-vector streaming sweeps
  * (even n1, 2^22 points or more): i3 chunks, prefetch distance and
- * narrow-sweep form (the slice width is fixed).  Host-only; SEDI_ERR_ARG on
- * bad values. */
+ * narrow-sweep form (the slice width is fixed).  Solves that run on chip use the
+ * period alone.  Host-only; SEDI_ERR_ARG on bad values. */
 int sedi_set_tuning(int solver, int precision, int batch, long n1, long n2, long n3, const int *choice);
 
 /*
@@ -399,8 +405,8 @@ double sedi_mixed_target(const sedi_ctx *ctx);
 /* Launch choices of a batched context: config[0..6] = lane-slice width, i3
  * chunks of a sweep, reliable-update period, iterations per captured graph,
  * lanes (padded right-hand sides), L2 prefetch distance in planes, form of
- * the narrow sweeps (see sedi_autotune).  SEDI_ERR_UNSUPPORTED for the
- * single-vector form. */
+ * the narrow sweeps (see sedi_autotune).  Where the solves run on chip the period
+ * alone acts.  SEDI_ERR_UNSUPPORTED for the single-vector form. */
 int sedi_ctx_config(const sedi_ctx *ctx, int *config);
 
 /*

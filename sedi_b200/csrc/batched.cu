@@ -3255,6 +3255,62 @@ static int tune_sweep_ms(sedi_ctx *h, double *ms_sum) {
 	return 0;
 }
 
+// A blocking seeded estimate on the context, timed.
+static int timed_estimate(Ctx *c, int batch, uint32_t seed, int maxiter, double tol, double *D, double *ms) {
+	const auto t0 = std::chrono::steady_clock::now();
+	const int rc = batched_estimate_src(c, batch, nullptr, seed, maxiter, tol, 1, D, nullptr, nullptr, nullptr, nullptr,
+	                                    nullptr);
+	*ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
+	return rc < 0 ? rc : 0;
+}
+
+// The autotuner where the solves run on chip: the sweeps' choices act on nothing
+// there, so only the reliable-update period is measured (with flags & 1, mixed).
+// *score_ms without flags & 1: an iteration of `batch` solves.
+static int autotune_on_chip(const TuneKey &key, int batch, int maxiter, double tol, uint32_t seed, int flags, int *out,
+                            double *score_ms) {
+	const bool mixed = key.precision == SEDI_PREC_MIXED;
+	const int ks = kernel_solver(key.solver, mixed);
+	Tuning best;
+	best.W = slice_for(key.R, !mixed, ks);
+	set_tuning(key, best);
+	int err = 0;
+	sedi_ctx *h = sedi_create(key.solver, (long)key.n1, (long)key.n2, (long)key.n3, 6.0, 1.0, 1.0, 0, key.precision,
+	                          batch, &err);
+	if (!h) return err ? err : SEDI_ERR_CUDA;
+	Batched *B = (Batched *)h->c.batched;
+	double *D = nullptr;
+	if (cudaMalloc(&D, sizeof(double) * h->c.g.n) != cudaSuccess) {
+		cudaGetLastError();
+		sedi_destroy(h);
+		return SEDI_ERR_NOMEM;
+	}
+	constexpr int kIterations = 20;
+	const bool solve = (flags & 1) != 0;
+	const int m = solve ? maxiter : kIterations;
+	const double t = solve ? tol : 0.0;
+	double best_ms = -1.0, ms = 0.0;
+	int rc = timed_estimate(&h->c, batch, seed, m, t, D, &ms);  // warm-up: loads the kernels
+	const int periods[] = {B->period, 20, 50};
+	for (int k = 0; k < (mixed && solve ? 3 : 1) && !rc; k++) {
+		B->period = periods[k];
+		if ((rc = timed_estimate(&h->c, batch, seed, m, t, D, &ms))) break;
+		if (best_ms < 0 || ms < best_ms) {
+			best_ms = ms;
+			if (mixed && solve) best.period = periods[k];
+		}
+	}
+	cudaFree(D);
+	sedi_destroy(h);
+	if (rc) return rc;
+	set_tuning(key, best);
+	const int form = default_form(ks, false);
+	const int choice[] = {best.W, best.nz, best.period, best.chunk, best.pfd, form};
+	for (int k = 0; k < 6; k++) out[k] = choice[k];
+	if (score_ms) *score_ms = solve ? best_ms : best_ms / kIterations;
+	return 0;
+}
+
 int batched_autotune(int solver, int precision, int batch, long long n1, long long n2, long long n3, int maxiter,
                      double tol, uint32_t seed, int flags, int *out, double *score_ms) {
 	const bool mixed = precision == SEDI_PREC_MIXED;
@@ -3267,6 +3323,9 @@ int batched_autotune(int solver, int precision, int batch, long long n1, long lo
 	if (single) flags &= ~1;
 	const int R = pick_R(batch, mixed);
 	const TuneKey key{solver, precision, R, n1, n2, n3};
+	const Geo geo{(int)n1, (int)n2, (int)n3, n1 * n2 * n3};
+	if (!single && resident_bytes(kernel_solver(solver, mixed), mixed, R, geo) > 0)
+		return autotune_on_chip(key, batch, maxiter, tol, seed, flags, out, score_ms);
 	std::vector<int> Ws;
 	if (single) {
 		Ws.push_back(2);
@@ -3350,13 +3409,7 @@ int batched_autotune(int solver, int precision, int batch, long long n1, long lo
 			sedi_destroy(h);
 			return SEDI_ERR_NOMEM;
 		}
-		auto timed = [&](double *ms) -> int {
-			const auto t0 = std::chrono::steady_clock::now();
-			const int rc = batched_estimate_src(c, batch, nullptr, seed, maxiter, tol, 1, D, nullptr, nullptr,
-			                                    nullptr, nullptr, nullptr);
-			*ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
-			return rc < 0 ? rc : 0;
-		};
+		auto timed = [&](double *ms) { return timed_estimate(c, batch, seed, maxiter, tol, D, ms); };
 		const int periods_mixed[] = {20, 32, 50}, period_fp64[] = {B->period};
 		const int *periods = mixed ? periods_mixed : period_fp64;
 		const int np = mixed ? 3 : 1;
