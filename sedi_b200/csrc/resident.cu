@@ -1,13 +1,15 @@
 // Resident solvers: whole Krylov solves in one cooperative launch, with the
 // fields of a right-hand side kept on chip (sm_100a).
 //
-// A grid of up to 148 x 16384 points has Krylov vectors that fit the
-// registers and shared memory of the GPU's 148 SMs.  A group of G blocks (one
-// per SM) then solves one right-hand side (FP64) or two (FP32, a float2 per
-// point): each block owns a box of rows x planes, all n1 points wide, with
-// the stencil input in shared memory (one ghost layer around it) and the
-// residual in registers.  An iteration moves no Krylov vector through HBM; x,
-// which no stencil reads, goes through L2.  CG's two reductions per iteration
+// A grid of up to 148 x 16384 points (CG) or 148 x 6144 (pipelined CG and
+// BiCGStab) has Krylov vectors that fit the registers and shared memory of the
+// GPU's 148 SMs, with some own-point fields in L2.  A group of G blocks (one per
+// SM; two in one box shape, for many small solves) then solves one right-hand
+// side (FP64) or two (FP32, a float2 per point): each block owns a box of rows x
+// planes, all n1 points wide, with the stencil input in shared memory (one ghost
+// layer around it) and the residual in registers.  An iteration moves no Krylov
+// vector through HBM; x, which no stencil reads, goes through L2.  CG's two
+// reductions per iteration
 // are the group's only two synchronisations: the one that ends an iteration
 // also publishes the boundary rows of the new residual, from which every
 // block forms its ghost points of the next direction itself.  With more
@@ -258,7 +260,7 @@ struct CgState {
 // p>; group sum; B: r -= alpha A p, boundary rows published; <r,u>, <r,r>;
 // group sum.
 //
-// 128^3 FP64: 128 blocks of 128 x 8 x 16 points (186 KB of shared memory, 64
+// 128^3 FP64: 144 blocks of 128 x 8 x 15 points (176 KB of shared memory, 64
 // registers of r per thread).
 // ---------------------------------------------------------------------------
 template <class V, int C, int D, int TMAX, int BLOCKS, bool UNIT>
@@ -1509,8 +1511,8 @@ size_t resident_bytes(int ks, bool fp32, int lanes, const Geo &g) {
 // A resident solver for up to `lanes` right-hand sides of the context's grid,
 // planned for `batch` of them; *out stays null where the grid or the device does
 // not take one (the streaming and march kernels serve those).  The caller gives
-// it *bytes of device memory, 16-byte aligned, with resident_bind: as the tail of
-// a vector, since an allocation of its own took 0.4 ms of a context's creation.
+// it *bytes of device memory, 16-byte aligned, with resident_bind: behind its
+// vectors, since an allocation of its own took 0.2-0.4 ms of a context's creation.
 int resident_alloc(Ctx *c, int ks, bool fp32, int lanes, int batch, Resident **out, size_t *bytes) {
 	*out = nullptr;
 	*bytes = 0;

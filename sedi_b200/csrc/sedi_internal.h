@@ -61,6 +61,7 @@ struct Ctx {
 	cudaStream_t own_stream;  // the context's own stream
 	int nblocks;
 
+	char *arena;  // the vectors below and the accumulators, then the on-chip solver's buffer
 	// single-vector FP64 buffers (n doubles each)
 	double *x, *b, *iM, *r, *rhat, *p[2], *v[2], *w[2], *u, *q, *s, *z;
 	double *partials;
