@@ -9,12 +9,11 @@
 // planes, all n1 points wide, with the stencil input in shared memory (one ghost
 // layer around it) and the residual in registers.  An iteration moves no Krylov
 // vector through HBM; x, which no stencil reads, goes through L2.  CG's two
-// reductions per iteration
-// are the group's only two synchronisations: the one that ends an iteration
-// also publishes the boundary rows of the new residual, from which every
-// block forms its ghost points of the next direction itself.  With more
-// right-hand sides than one group needs blocks for, groups run side by side
-// and take them in turn.
+// reductions per iteration are the group's only two synchronisations: the one
+// that ends an iteration also publishes the boundary rows of the new residual,
+// from which every block forms its ghost points of the next direction itself.
+// With more right-hand sides than one group needs blocks for, groups run side by
+// side and take them in turn.
 //
 // Elementwise values round as the sweeps of the other forms: FP64 operator by
 // operator as the reference (Cg.hpp:107-207), FP32 with the products fused
@@ -1315,11 +1314,11 @@ size_t buffer_bytes(int ks, int shape, int G, int groups, int nd, int RG, int n1
 
 // Plan with the smallest estimated time of an iteration of `units` solves, and
 // that time in cycles; *most grows to the buffer of any plan for at most `units`
-// solves.  Measured on B200 (FP64, 1.95 GHz) before the ghost rows
-// came from a table, which took 1500-6000 cycles off every CG shape alike
-// (16384 points now 32000): the two reductions,
-// ghost rows and launch of each phase take 9000-11000 cycles between blocks;
-// a point adds 1.3 where A p stays in registers (2048 points a block 13600, 8192
+// solves.  Measured on B200 (FP64, 1.95 GHz) before the ghost rows came from a
+// table, which took 1500-6000 cycles off every CG shape alike (16384 points now
+// 32000; the rule against the streaming sweeps is that much on their side): the
+// two reductions, ghost rows and launch of each phase take 9000-11000 cycles
+// between blocks; a point adds 1.3 where A p stays in registers (2048 points a block 13600, 8192
 // 20100), 1.65 with two stencil passes (16384: 38000), 1.8 at three rows a
 // thread (12672: 32500), and 3.2 with two blocks on an SM (2 x 8192: 37400).
 // Pipelined CG: 256 points a block 7700, 2048 10400, 4096 14000; BiCGStab: 512
@@ -1490,9 +1489,10 @@ static bool resident_takes(int ks, bool fp32, int lanes, const Geo &g, int sms, 
 	// lane (conversions for its FP64 sums, less since the ghost table); at 1.6 no
 	// measured batch goes on chip that is slower there (us an iteration, on chip and
 	// streaming: 80^3 x 32 110 / 133; 96^3 x 16 105 / 99, 96^3 x 32 208 / 168,
-	// 128^3 x 16 230 / 201; 64^3 x 64, 107 / 115, and 80^3 x 64, 221 / 240, stream).  One right-hand side has no streaming
-	// form at these sizes (its march kernels take 11.7 us an iteration at 32^3, 47
-	// at 128^3; this 5.5 and 16.4), a batch does.
+	// 128^3 x 16 230 / 201); two that would gain 7% stream (64^3 x 64, 107 / 115,
+	// and 80^3 x 64, 221 / 240).  One right-hand side has no streaming form at
+	// these sizes (its march kernels take 11.7 us an iteration at 32^3, 47 at
+	// 128^3; this 5.5 and 16.4), a batch does.
 	if (fp32) cycles *= 1.6;
 	return lanes <= 1 || cycles <= stream_cycles(ks, g, lanes, fp32);
 }

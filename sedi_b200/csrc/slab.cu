@@ -13,10 +13,10 @@
 //
 // Dot products are returned per plane, each summed in a fixed order that
 // depends only on n1 and n2 (the plane is cut into kSlabChunks row chunks, a
-// cluster of kSlabSplit blocks each, then the chunks are added in a fixed tree), so a plane's partial
-// sum is the same whichever rank holds the plane; the planes are then added in
-// an order fixed by their number (k_slab_totals).  The solution therefore does not depend on the number of
-// slabs, bit for bit.  Elementwise values round as the reference's
+// cluster of kSlabSplit blocks each, then the chunks are added in a fixed tree),
+// so a plane's partial sum is the same whichever rank holds the plane; the planes
+// are then added in an order fixed by their number (k_slab_totals).  The solution
+// therefore does not depend on the number of slabs, bit for bit.  Elementwise values round as the reference's
 // (operator by operator, no FMA contraction), like the single-vector form:
 // a stencil input the reference stores (u = r .* iM, m = w .* iM, p_hat,
 // s_hat) is formed at each neighbour read with the same rounding.
