@@ -754,31 +754,38 @@ int plain_solve_resident(Ctx *c, bool vim, int maxiter, double tol, double *fina
 	return solve_impl<false>(c, im, maxiter, tol, final_err, final_iter);
 }
 
-// Whether a kernel may take the caller's vector as it is: aligned, and wholly
-// inside one cudaMalloc'ed block of the context's GPU.  Anything else (pool,
+// Whether a kernel may take the caller's vectors as they are: aligned, and each
+// wholly inside one cudaMalloc'ed block of the context's GPU.  Anything else (pool,
 // mapped or managed memory, pinned host memory, another GPU, 4-byte aligned) goes
 // by way of a copy, which takes what CUDA takes and refuses the rest with an
-// error, where a kernel would fault.  0.5 us a vector.
-static bool in_place(const Ctx *c, const void *p, size_t bytes) {
+// error, where a kernel would fault.  A query takes 0.45 us; vectors of one block
+// (a caching allocator's, say) need one.
+static bool in_place(const Ctx *c, const void *p, const void *q, size_t bytes) {
 	typedef CUresult (*AttrFn)(unsigned, CUpointer_attribute *, void **, CUdeviceptr);
 	static const AttrFn fn = []() -> AttrFn {
 		void *f = nullptr;
-		cudaDriverEntryPointQueryResult q;
-		if (cudaGetDriverEntryPoint("cuPointerGetAttributes", &f, cudaEnableDefault, &q) == cudaSuccess &&
-		    q == cudaDriverEntryPointSuccess)
+		cudaDriverEntryPointQueryResult r;
+		if (cudaGetDriverEntryPoint("cuPointerGetAttributes", &f, cudaEnableDefault, &r) == cudaSuccess &&
+		    r == cudaDriverEntryPointSuccess)
 			return (AttrFn)f;
 		cudaGetLastError();
 		return nullptr;
 	}();
-	if (!fn || (uintptr_t)p % sizeof(double) != 0) return false;
-	unsigned long long type = 0, device = 0, managed = 0, block = 0, start = 0, size = 0;  // block: cudaMalloc'ed, so mapped all over
-	CUpointer_attribute what[] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE,      CU_POINTER_ATTRIBUTE_DEVICE_ORDINAL,
-	                              CU_POINTER_ATTRIBUTE_IS_MANAGED,       CU_POINTER_ATTRIBUTE_IS_LEGACY_CUDA_IPC_CAPABLE,
-	                              CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, CU_POINTER_ATTRIBUTE_RANGE_SIZE};
-	void *into[] = {&type, &device, &managed, &block, &start, &size};
-	if (fn(6, what, into, (CUdeviceptr)p) != CUDA_SUCCESS) return false;
-	return type == CU_MEMORYTYPE_DEVICE && !managed && block && (int)device == c->device &&
-	       (unsigned long long)(uintptr_t)p + bytes <= start + size;
+	unsigned long long start = 0, size = 0;
+	for (const void *v : {p, q}) {
+		const unsigned long long at = (uintptr_t)v;
+		if (!fn || at % sizeof(double) != 0) return false;
+		if (size && at >= start && at + bytes <= start + size) continue;
+		unsigned long long type = 0, device = 0, managed = 0, block = 0;  // block: cudaMalloc'ed, so mapped all over
+		CUpointer_attribute what[] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE,      CU_POINTER_ATTRIBUTE_DEVICE_ORDINAL,
+		                              CU_POINTER_ATTRIBUTE_IS_MANAGED,       CU_POINTER_ATTRIBUTE_IS_LEGACY_CUDA_IPC_CAPABLE,
+		                              CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+		void *into[] = {&type, &device, &managed, &block, &start, &size};
+		if (fn(6, what, into, (CUdeviceptr)at) != CUDA_SUCCESS || type != CU_MEMORYTYPE_DEVICE || managed || !block ||
+		    (int)device != c->device || at < start || at + bytes > start + size)
+			return false;
+	}
+	return true;
 }
 
 int plain_solve_dev(Ctx *c, const double *b, double *x, const double *iM, int maxiter, double tol,
@@ -787,7 +794,7 @@ int plain_solve_dev(Ctx *c, const double *b, double *x, const double *iM, int ma
 	cudaStream_t s = c->stream;
 	// On chip the solve reads b and x once, before it first writes x (b and x may
 	// overlap), and needs no copies of them.
-	if (!iM && c->res && in_place(c, b, bytes) && in_place(c, x, bytes))
+	if (!iM && c->res && in_place(c, b, x, bytes))
 		return resident_solve(c, b, x, maxiter, tol, final_err, final_iter);
 	SEDI_TRY(cudaMemcpyAsync(c->b, b, bytes, cudaMemcpyDeviceToDevice, s));
 	SEDI_TRY(cudaMemcpyAsync(c->x, x, bytes, cudaMemcpyDeviceToDevice, s));
